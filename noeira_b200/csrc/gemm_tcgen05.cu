@@ -5,8 +5,8 @@
 //     64-wide k-block; tcgen05.commit releases the stage / publishes the accumulator;
 //   * persistent CTAs (one per SM) walk the tile list; two TMEM accumulators let the epilogue
 //     of tile i overlap the main loop of tile i+1;
-//   * warp roles (192 threads): warp 0 = TMA producer, warp 1 = MMA issuer + TMEM owner,
-//     warps 2..5 = epilogue (TMEM quarter = warp_id % 4);
+//   * warp roles (320 threads): warp 0 = TMA producer, warp 1 = MMA issuer + TMEM owner,
+//     warps 2..9 = epilogue (TMEM quarter = warp_id % 4, two warps per quarter);
 //   * both operands may be K-major ([rows, K] row-major) or MN-major ([K, rows] row-major), so
 //     forward (x·W, W stored [IN, OUT]), dgrad (dy·Wᵀ) and wgrad (xᵀ·dy) all run from the
 //     natural layouts without a transpose pass;
@@ -30,7 +30,11 @@ using namespace nb;
 constexpr int BM = 128;
 constexpr int BK = 64;  // 64 bf16 = 128 bytes = one swizzle row
 constexpr int UMMA_K = 16;
-constexpr int NUM_THREADS = 192;
+// Eight epilogue warps: two share a 32-row quarter of the accumulator and take its column groups in turn.  With four the
+// epilogue of a 256 x 256 tile (bias, GELU, residual, bf16 store) took longer than the twelve k-blocks of K = 768, and the
+// tensor core waited for a free accumulator: 24576 x 3072 x 768 with GELU took 240 us, 176 us with eight.
+constexpr int EPI_WARPS = 8;
+constexpr int NUM_THREADS = 64 + 32 * EPI_WARPS;
 
 struct GemmParams {
   int M, N, K;
@@ -169,13 +173,78 @@ __device__ __forceinline__ void epilogue_prefetch16(const GemmParams& p, int row
   }
 }
 
-__device__ __forceinline__ void epilogue_store16(const GemmParams& p, int row, int col0, float (&v)[16],
-                                                 const EpiPrefetch& pf) {
+// alpha, bias and activation of 16 consecutive columns; `sv`: the 16 values of the saved / residual tensor when dact is set.
+// The bias comes from the lanes that hold it (see load_bias): lane b0 + j has columns 4j .. 4j + 3 of the chunk.
+__device__ __forceinline__ void epilogue_math16(const GemmParams& p, const float4& bias, int b0, float (&v)[16], const float (&sv)[16]) {
 #pragma unroll
   for (int j = 0; j < 16; ++j) v[j] *= p.alpha;
-  const bool full = (col0 + 16 <= p.N);
   if (p.bias) {
-    if (full && (col0 % 4 == 0)) {
+#pragma unroll
+    for (int j = 0; j < 4; ++j) {
+      v[4 * j] += __shfl_sync(0xffffffffu, bias.x, b0 + j);
+      v[4 * j + 1] += __shfl_sync(0xffffffffu, bias.y, b0 + j);
+      v[4 * j + 2] += __shfl_sync(0xffffffffu, bias.z, b0 + j);
+      v[4 * j + 3] += __shfl_sync(0xffffffffu, bias.w, b0 + j);
+    }
+  }
+  if (p.act) act_apply16(p.act, v);
+  if (p.dact) dact_apply16(p.dact, v, sv);
+}
+// The bias of a warp's column groups (`half`, `half` + 2, ... of G columns each; at most 128 columns), four per lane, fetched
+// while the accumulator is still being computed.  Loaded inside the chunk loop it cost an L2 round trip per 16 columns (most
+// of the L1 is shared memory here): 24576 x 2304 x 768 took 101 us with it and 77 us without a bias.
+template <int BN, int G>
+__device__ __forceinline__ float4 load_bias(const GemmParams& p, int n0, int half, int lane) {
+  float4 b = make_float4(0.f, 0.f, 0.f, 0.f);
+  const int idx = 4 * lane, c = half * G + idx / G * 2 * G + idx % G, col = n0 + c;
+  if (p.bias && c < BN) {
+    if (col < p.N) b.x = p.bias[col];
+    if (col + 1 < p.N) b.y = p.bias[col + 1];
+    if (col + 2 < p.N) b.z = p.bias[col + 2];
+    if (col + 3 < p.N) b.w = p.bias[col + 3];
+  }
+  return b;
+}
+__device__ __forceinline__ void unpack16(const uint4 (&w)[2], float (&f)[16]) {
+  const __nv_bfloat162* h0 = reinterpret_cast<const __nv_bfloat162*>(&w[0]);
+  const __nv_bfloat162* h1 = reinterpret_cast<const __nv_bfloat162*>(&w[1]);
+#pragma unroll
+  for (int j = 0; j < 4; ++j) {
+    f[2 * j] = __low2float(h0[j]);
+    f[2 * j + 1] = __high2float(h0[j]);
+    f[8 + 2 * j] = __low2float(h1[j]);
+    f[8 + 2 * j + 1] = __high2float(h1[j]);
+  }
+}
+__device__ __forceinline__ uint4 pack8f(const float* v) {
+  uint4 pk;
+  __nv_bfloat162 h0 = __floats2bfloat162_rn(v[0], v[1]), h1 = __floats2bfloat162_rn(v[2], v[3]),
+                 h2 = __floats2bfloat162_rn(v[4], v[5]), h3 = __floats2bfloat162_rn(v[6], v[7]);
+  pk.x = *reinterpret_cast<uint32_t*>(&h0);
+  pk.y = *reinterpret_cast<uint32_t*>(&h1);
+  pk.z = *reinterpret_cast<uint32_t*>(&h2);
+  pk.w = *reinterpret_cast<uint32_t*>(&h3);
+  return pk;
+}
+
+// direct store of 16 columns by the thread that owns them (second phase of a split-K GEMM)
+__device__ __forceinline__ void epilogue_store16(const GemmParams& p, int row, int col0, float (&v)[16],
+                                                 const EpiPrefetch& pf) {
+  const bool full = (col0 + 16 <= p.N);
+  float sv[16];
+  if (p.dact) {
+    if (full && (p.ld_aux % 8 == 0)) {
+      unpack16(pf.aux, sv);
+    } else {
+      const __nv_bfloat16* ax = p.aux + (size_t)row * p.ld_aux + col0;
+#pragma unroll
+      for (int j = 0; j < 16; ++j) sv[j] = (col0 + j < p.N) ? __bfloat162float(ax[j]) : 0.f;
+    }
+  }
+#pragma unroll
+  for (int j = 0; j < 16; ++j) v[j] *= p.alpha;
+  if (p.bias) {
+    if (full) {
 #pragma unroll
       for (int j = 0; j < 16; j += 4) {
         const float4 bv = __ldg(reinterpret_cast<const float4*>(p.bias + col0 + j));
@@ -188,25 +257,7 @@ __device__ __forceinline__ void epilogue_store16(const GemmParams& p, int row, i
     }
   }
   if (p.act) act_apply16(p.act, v);
-  if (p.dact) {
-    float sv[16];
-    if (full && (p.ld_aux % 8 == 0)) {
-      const __nv_bfloat162* h0 = reinterpret_cast<const __nv_bfloat162*>(&pf.aux[0]);
-      const __nv_bfloat162* h1 = reinterpret_cast<const __nv_bfloat162*>(&pf.aux[1]);
-#pragma unroll
-      for (int j = 0; j < 4; ++j) {
-        sv[2 * j] = __low2float(h0[j]);
-        sv[2 * j + 1] = __high2float(h0[j]);
-        sv[8 + 2 * j] = __low2float(h1[j]);
-        sv[8 + 2 * j + 1] = __high2float(h1[j]);
-      }
-    } else {
-      const __nv_bfloat16* ax = p.aux + (size_t)row * p.ld_aux + col0;
-#pragma unroll
-      for (int j = 0; j < 16; ++j) sv[j] = (col0 + j < p.N) ? __bfloat162float(ax[j]) : 0.f;
-    }
-    dact_apply16(p.dact, v, sv);
-  }
+  if (p.dact) dact_apply16(p.dact, v, sv);
   if (p.out_f32) {
     float* o = reinterpret_cast<float*>(p.D) + (size_t)row * p.ldd + col0;
     if (full && (p.ldd % 4 == 0)) {
@@ -228,21 +279,183 @@ __device__ __forceinline__ void epilogue_store16(const GemmParams& p, int row, i
     __nv_bfloat16* o = reinterpret_cast<__nv_bfloat16*>(p.D) + (size_t)row * p.ldd + col0;
     if (full && (p.ldd % 8 == 0)) {
 #pragma unroll
-      for (int j = 0; j < 16; j += 8) {
-        uint4 pk;
-        __nv_bfloat162 h0 = __floats2bfloat162_rn(v[j], v[j + 1]), h1 = __floats2bfloat162_rn(v[j + 2], v[j + 3]),
-                       h2 = __floats2bfloat162_rn(v[j + 4], v[j + 5]), h3 = __floats2bfloat162_rn(v[j + 6], v[j + 7]);
-        pk.x = *reinterpret_cast<uint32_t*>(&h0);
-        pk.y = *reinterpret_cast<uint32_t*>(&h1);
-        pk.z = *reinterpret_cast<uint32_t*>(&h2);
-        pk.w = *reinterpret_cast<uint32_t*>(&h3);
-        *reinterpret_cast<uint4*>(o + j) = pk;
-      }
+      for (int j = 0; j < 16; j += 8) *reinterpret_cast<uint4*>(o + j) = pack8f(v + j);
     } else {
 #pragma unroll
       for (int j = 0; j < 16; ++j)
         if (col0 + j < p.N) o[j] = __float2bfloat16(v[j]);
     }
+  }
+}
+
+// Epilogue of one warp: rows [row0, row0 + 32) of the tile (lane = row), column groups `half`, `half` + 2, ... of the tile's
+// BN columns that start at column n0 of the output.
+//
+// Tensor memory hands every lane a whole row, and a store straight from there touches 32 rows with 16 bytes each: 32 L2
+// requests per instruction, which made GEMMs with K <= 1024 epilogue-bound (24576 x 2304 x 768 with bias: 142 us with direct
+// stores from four warps, 105 us from eight, 101 us staged, 82 us with the bias fetched ahead, see load_bias).  So a group goes through 4 KB of shared memory per warp: the lane that
+// owns the row does the arithmetic and writes its packed row (16-byte chunks XOR-swizzled, no bank conflicts), then the warp
+// copies the group out with whole 64- or 128-byte row segments per request.  The saved / residual tensor comes in the same
+// way in front of the arithmetic, the old fp32 output is added during the copy.
+constexpr int EPI_STAGE_BYTES = 4096;   // per warp
+
+// byte offset of 16-byte chunk `ch` of row `r`; CPR = chunks per row (8: 128-byte rows, 4: 64-byte rows)
+template <int CPR>
+__device__ __forceinline__ int epi_off(int r, int ch) {
+  return CPR == 8 ? r * 128 + ((ch ^ (r & 7)) << 4) : r * 64 + ((ch ^ ((r >> 1) & 3)) << 4);
+}
+
+template <int BN>
+__host__ __device__ constexpr int epi_group() { return BN >= 128 ? 64 : 32; }   // columns per group, bf16 output
+template <int BN>
+__device__ __forceinline__ void epilogue_tile_bf16(const GemmParams& p, const float4& bias, uint32_t taddr, uint8_t* st, int row0,
+                                                   int n0, int half, int lane) {
+  constexpr int G = epi_group<BN>(), CPR = G / 8, NV = CPR;   // columns per group; 16-byte vectors per lane and group
+  constexpr int NC = (BN < G ? BN : G) / 16;                      // 16-column chunks per group
+  constexpr int RS = 32 / CPR;                                    // rows per copy instruction
+  const int rr0 = lane / CPR, ch = lane % CPR;                    // copies: this lane's first row and its chunk of every row
+  const bool vec_d = p.ldd % 8 == 0, vec_a = p.ld_aux % 8 == 0;
+  uint4 ax[NV];
+  auto load_aux = [&](int c) {
+    const int col = n0 + c + ch * 8;
+    const __nv_bfloat16* a = p.aux + (size_t)(row0 + rr0) * p.ld_aux + col;
+#pragma unroll
+    for (int i = 0; i < NV; ++i) {
+      ax[i] = make_uint4(0, 0, 0, 0);
+      if (row0 + rr0 + i * RS < p.M && col < p.N) {
+        if (vec_a && col + 8 <= p.N) {
+          ax[i] = __ldg(reinterpret_cast<const uint4*>(a));
+        } else {
+          __nv_bfloat16 e[8];
+#pragma unroll
+          for (int j = 0; j < 8; ++j) e[j] = col + j < p.N ? a[j] : __float2bfloat16(0.f);
+          ax[i] = *reinterpret_cast<const uint4*>(e);
+        }
+      }
+      a += (size_t)RS * p.ld_aux;
+    }
+  };
+  if (p.dact && half * G < BN && n0 + half * G < p.N) load_aux(half * G);
+#pragma unroll 1
+  for (int c = half * G; c < BN && n0 + c < p.N; c += 2 * G) {
+    if (p.dact) {
+#pragma unroll
+      for (int i = 0; i < NV; ++i) *reinterpret_cast<uint4*>(st + epi_off<CPR>(rr0 + i * RS, ch)) = ax[i];
+      __syncwarp();
+      if (c + 2 * G < BN && n0 + c + 2 * G < p.N) load_aux(c + 2 * G);
+    }
+#pragma unroll 1
+    for (int k = 0; k < NC; ++k) {
+      uint32_t r[16];
+      tmem_ld_32x32b_x16(taddr + (uint32_t)(c + 16 * k), r);
+      tmem_ld_wait();
+      float v[16], sv[16];
+#pragma unroll
+      for (int j = 0; j < 16; ++j) v[j] = __uint_as_float(r[j]);
+      uint8_t* s0 = st + epi_off<CPR>(lane, 2 * k);
+      uint8_t* s1 = st + epi_off<CPR>(lane, 2 * k + 1);
+      if (p.dact) {
+        const uint4 w[2] = {*reinterpret_cast<const uint4*>(s0), *reinterpret_cast<const uint4*>(s1)};
+        unpack16(w, sv);
+      }
+      epilogue_math16(p, bias, ((c / (2 * G)) * G + 16 * k) >> 2, v, sv);
+      *reinterpret_cast<uint4*>(s0) = pack8f(v);
+      *reinterpret_cast<uint4*>(s1) = pack8f(v + 8);
+    }
+    __syncwarp();
+    const int col = n0 + c + ch * 8;
+    __nv_bfloat16* o = reinterpret_cast<__nv_bfloat16*>(p.D) + (size_t)(row0 + rr0) * p.ldd + col;
+    const int rows = (col < p.N && ch * 8 < BN) ? p.M - row0 : 0;
+    if (vec_d && col + 8 <= p.N) {
+#pragma unroll
+      for (int i = 0; i < NV; ++i) {
+        if (rr0 + i * RS < rows) *reinterpret_cast<uint4*>(o) = *reinterpret_cast<const uint4*>(st + epi_off<CPR>(rr0 + i * RS, ch));
+        o += (size_t)RS * p.ldd;
+      }
+    } else {
+#pragma unroll 1
+      for (int i = 0; i < NV; ++i) {
+        const uint4 w = *reinterpret_cast<const uint4*>(st + epi_off<CPR>(rr0 + i * RS, ch));
+        const __nv_bfloat16* e = reinterpret_cast<const __nv_bfloat16*>(&w);
+#pragma unroll
+        for (int j = 0; j < 8; ++j)
+          if (rr0 + i * RS < rows && col + j < p.N) o[j] = e[j];
+        o += (size_t)RS * p.ldd;
+      }
+    }
+    __syncwarp();
+  }
+}
+
+// fp32 output, or (split) the raw fp32 partial tile of a split-K item at `part` (row pitch BN)
+template <int BN>
+__device__ __forceinline__ void epilogue_tile_f32(const GemmParams& p, const float4& bias, uint32_t taddr, uint8_t* st, int row0,
+                                                  int n0, int half, int lane, float* part) {
+  constexpr int G = 32;
+  constexpr int NC = (BN < G ? BN : G) / 16;
+  const bool vec_d = p.ldd % 4 == 0;
+#pragma unroll 1
+  for (int c = half * G; c < BN && n0 + c < p.N; c += 2 * G) {
+#pragma unroll 1
+    for (int k = 0; k < NC; ++k) {
+      uint32_t r[16];
+      tmem_ld_32x32b_x16(taddr + (uint32_t)(c + 16 * k), r);
+      tmem_ld_wait();
+      float v[16];
+#pragma unroll
+      for (int j = 0; j < 16; ++j) v[j] = __uint_as_float(r[j]);
+      const int col0 = n0 + c + 16 * k;
+      if (!part) {
+        float sv[16];
+        if (p.dact) {
+          const __nv_bfloat16* ax = p.aux + (size_t)(row0 + lane) * p.ld_aux + col0;
+#pragma unroll
+          for (int j = 0; j < 16; ++j) sv[j] = (row0 + lane < p.M && col0 + j < p.N) ? __bfloat162float(ax[j]) : 0.f;
+        }
+        epilogue_math16(p, bias, ((c / (2 * G)) * G + 16 * k) >> 2, v, sv);
+      }
+#pragma unroll
+      for (int j = 0; j < 4; ++j)
+        *reinterpret_cast<float4*>(st + epi_off<8>(lane, 4 * k + j)) = make_float4(v[4 * j], v[4 * j + 1], v[4 * j + 2], v[4 * j + 3]);
+    }
+    __syncwarp();
+    const int rr0 = lane >> 3, ch = lane & 7, col = n0 + c + ch * 4;
+    if (part) {
+      float* o = part + (size_t)rr0 * BN + c + ch * 4;
+#pragma unroll
+      for (int i = 0; i < 8; ++i)
+        if (ch * 4 < BN) *reinterpret_cast<float4*>(o + (size_t)i * 4 * BN) = *reinterpret_cast<const float4*>(st + epi_off<8>(rr0 + 4 * i, ch));
+    } else {
+      float* o = reinterpret_cast<float*>(p.D) + (size_t)(row0 + rr0) * p.ldd + col;
+      const int rows = (col < p.N && ch * 4 < BN) ? p.M - row0 : 0;
+      if (vec_d && col + 4 <= p.N) {
+#pragma unroll 1
+        for (int h = 0; h < 8; h += 4) {      // four rows of this lane at a time: their old values are in flight together
+          float4 old[4];
+#pragma unroll
+          for (int i = 0; i < 4; ++i)
+            if (p.accumulate && rr0 + 4 * (h + i) < rows) old[i] = *reinterpret_cast<const float4*>(o + (size_t)i * 4 * p.ldd);
+#pragma unroll
+          for (int i = 0; i < 4; ++i) {
+            float4 w = *reinterpret_cast<const float4*>(st + epi_off<8>(rr0 + 4 * (h + i), ch));
+            if (p.accumulate) { w.x += old[i].x; w.y += old[i].y; w.z += old[i].z; w.w += old[i].w; }
+            if (rr0 + 4 * (h + i) < rows) *reinterpret_cast<float4*>(o + (size_t)i * 4 * p.ldd) = w;
+          }
+          o += (size_t)16 * p.ldd;
+        }
+      } else {
+#pragma unroll 1
+        for (int i = 0; i < 8; ++i) {
+          const float4 w = *reinterpret_cast<const float4*>(st + epi_off<8>(rr0 + 4 * i, ch));
+          const float e[4] = {w.x, w.y, w.z, w.w};
+#pragma unroll
+          for (int j = 0; j < 4; ++j)
+            if (rr0 + 4 * i < rows && col + j < p.N) o[j] = p.accumulate ? o[j] + e[j] : e[j];
+          o += (size_t)4 * p.ldd;
+        }
+      }
+    }
+    __syncwarp();
   }
 }
 
@@ -268,7 +481,8 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
 
   extern __shared__ __align__(1024) uint8_t smem_raw[];
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
-  uint64_t* full_bar = reinterpret_cast<uint64_t*>(smem + STAGES * STAGE_BYTES);
+  uint8_t* epi_stage = smem + STAGES * STAGE_BYTES;
+  uint64_t* full_bar = reinterpret_cast<uint64_t*>(epi_stage + EPI_WARPS * EPI_STAGE_BYTES);
   uint64_t* empty_bar = full_bar + STAGES;
   uint64_t* tfull_bar = empty_bar + STAGES;
   uint64_t* tempty_bar = tfull_bar + 2;
@@ -287,7 +501,7 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
     }
     for (int a = 0; a < 2; ++a) {
       mbar_init(&tfull_bar[a], 1);
-      mbar_init(&tempty_bar[a], 4);
+      mbar_init(&tempty_bar[a], EPI_WARPS);
     }
     *abort_flag = 0;
     fence_barrier_init();
@@ -415,8 +629,8 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
       }
     }
   } else {
-    // ------------------------------------------------------------------ epilogue (warps 2..5)
-    const int quarter = warp & 3;
+    // ------------------------------------------------------------------ epilogue (warps 2..9)
+    const int quarter = warp & 3, half = (warp - 2) >> 2;
     int acc = 0;
     uint32_t acc_phase = 0;
     bool ok = true;
@@ -424,51 +638,22 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
       int mb, nb_;
       const int tile = item / p.splits;
       tile_coords(tile, p.tiles_m, p.tiles_n, mb, nb_);
+      const float4 bias = p.out_f32 ? load_bias<BN, 32>(p, nb_ * BN, half, lane) : load_bias<BN, epi_group<BN>()>(p, nb_ * BN, half, lane);
       if (*abort_flag || !mbar_wait(&tfull_bar[acc], acc_phase, p.status, 4)) { ok = false; *abort_flag = 1; break; }
       tc_fence_after();
-      const int row_in_tile = quarter * 32 + lane;
-      const int row = mb * BM + row_in_tile;
-      const bool row_ok = row < p.M;
-      const uint32_t taddr0 = tmem_base + ((uint32_t)(quarter * 32) << 16) + (uint32_t)(acc * BN);
-      if (p.splits == 1) {
-        // rolled on purpose (one copy of the chunk body in the instruction cache); the chunk's global loads
-        // (saved activation, old output) are issued one chunk ahead of their use
-        EpiPrefetch pf;
-        epilogue_prefetch16(p, row, nb_ * BN, row_ok, pf);
-#pragma unroll 1
-        for (int c0 = 0; c0 < BN; c0 += 16) {
-          uint32_t r[16];
-          tmem_ld_32x32b_x16(taddr0 + (uint32_t)c0, r);
-          const EpiPrefetch cur = pf;
-          if (c0 + 16 < BN) epilogue_prefetch16(p, row, nb_ * BN + c0 + 16, row_ok, pf);
-          tmem_ld_wait();
-          const int col0 = nb_ * BN + c0;
-          if (row_ok && col0 < p.N) {
-            float v[16];
-#pragma unroll
-            for (int j = 0; j < 16; ++j) v[j] = __uint_as_float(r[j]);
-            epilogue_store16(p, row, col0, v, cur);
-          }
-        }
-        tc_fence_before();
-        __syncwarp();
-        if (lane == 0) mbar_arrive(&tempty_bar[acc]);
-      } else {
-        // split-K: park the fp32 partial tile; splitk_reduce_kernel sums the splits in index order afterwards
-        float* wtile = p.ws + (size_t)item * (BM * BN) + (size_t)row_in_tile * BN;
-#pragma unroll 1
-        for (int c0 = 0; c0 < BN; c0 += 16) {
-          uint32_t r[16];
-          tmem_ld_32x32b_x16(taddr0 + (uint32_t)c0, r);
-          tmem_ld_wait();
-#pragma unroll
-          for (int j = 0; j < 16; j += 4)
-            *reinterpret_cast<uint4*>(wtile + c0 + j) = make_uint4(r[j], r[j + 1], r[j + 2], r[j + 3]);
-        }
-        tc_fence_before();
-        __syncwarp();
-        if (lane == 0) mbar_arrive(&tempty_bar[acc]);
-      }
+      const int row_in_tile = quarter * 32;
+      const uint32_t taddr0 = tmem_base + ((uint32_t)row_in_tile << 16) + (uint32_t)(acc * BN);
+      uint8_t* st = epi_stage + (warp - 2) * EPI_STAGE_BYTES;
+      if (p.splits > 1)   // park the fp32 partial tile; splitk_reduce_kernel sums the splits in index order afterwards
+        epilogue_tile_f32<BN>(p, bias, taddr0, st, mb * BM + row_in_tile, nb_ * BN, half, lane,
+                              p.ws + (size_t)item * (BM * BN) + (size_t)row_in_tile * BN);
+      else if (p.out_f32)
+        epilogue_tile_f32<BN>(p, bias, taddr0, st, mb * BM + row_in_tile, nb_ * BN, half, lane, nullptr);
+      else
+        epilogue_tile_bf16<BN>(p, bias, taddr0, st, mb * BM + row_in_tile, nb_ * BN, half, lane);
+      tc_fence_before();
+      __syncwarp();
+      if (lane == 0) mbar_arrive(&tempty_bar[acc]);
       if (++acc == 2) { acc = 0; acc_phase ^= 1u; }
     }
   }
@@ -546,7 +731,8 @@ gemm2_bf16_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant
 
   extern __shared__ __align__(1024) uint8_t smem_raw[];
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
-  uint64_t* full_bar = reinterpret_cast<uint64_t*>(smem + STAGES2 * STAGE_BYTES);   // used in the leader only
+  uint8_t* epi_stage = smem + STAGES2 * STAGE_BYTES;
+  uint64_t* full_bar = reinterpret_cast<uint64_t*>(epi_stage + EPI_WARPS * EPI_STAGE_BYTES);   // used in the leader only
   uint64_t* empty_bar = full_bar + STAGES2;
   uint64_t* tfull_bar = empty_bar + STAGES2;
   uint64_t* tempty_bar = tfull_bar + 2;                                             // used in the leader only
@@ -566,7 +752,7 @@ gemm2_bf16_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant
     }
     for (int a = 0; a < 2; ++a) {
       mbar_init(&tfull_bar[a], 1);
-      mbar_init(&tempty_bar[a], 8);   // four epilogue warps in each CTA
+      mbar_init(&tempty_bar[a], 2 * EPI_WARPS);   // the epilogue warps of both CTAs
     }
     *abort_flag = 0;
     fence_barrier_init();
@@ -652,36 +838,22 @@ gemm2_bf16_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant
       }
     }
   } else {
-    // ------------------------------------------------------------------ epilogue (warps 2..5 of both CTAs)
-    const int quarter = warp & 3;
+    // ------------------------------------------------------------------ epilogue (warps 2..9 of both CTAs)
+    const int quarter = warp & 3, half = (warp - 2) >> 2;
     int acc = 0;
     uint32_t acc_phase = 0;
     bool ok = true;
     for (int tile = cluster_id; tile < num_tiles && ok; tile += num_clusters) {
       int mb, nb_;
       tile_coords(tile, p.tiles_m, p.tiles_n, mb, nb_);
+      const float4 bias = p.out_f32 ? load_bias<BN2, 32>(p, nb_ * BN2, half, lane) : load_bias<BN2, epi_group<BN2>()>(p, nb_ * BN2, half, lane);
       if (*abort_flag || !mbar_wait(&tfull_bar[acc], acc_phase, p.status, 24)) { ok = false; *abort_flag = 1; break; }
       tc_fence_after();
-      const int row = mb * (2 * BM) + (int)rank * BM + quarter * 32 + lane;
-      const bool row_ok = row < p.M;
+      const int row0 = mb * (2 * BM) + (int)rank * BM + quarter * 32;
       const uint32_t taddr0 = tmem_base + ((uint32_t)(quarter * 32) << 16) + (uint32_t)(acc * BN2);
-      EpiPrefetch pf;
-      epilogue_prefetch16(p, row, nb_ * BN2, row_ok, pf);
-#pragma unroll 1
-      for (int c0 = 0; c0 < BN2; c0 += 16) {
-        uint32_t r[16];
-        tmem_ld_32x32b_x16(taddr0 + (uint32_t)c0, r);
-        const EpiPrefetch cur = pf;
-        if (c0 + 16 < BN2) epilogue_prefetch16(p, row, nb_ * BN2 + c0 + 16, row_ok, pf);
-        tmem_ld_wait();
-        const int col0 = nb_ * BN2 + c0;
-        if (row_ok && col0 < p.N) {
-          float v[16];
-#pragma unroll
-          for (int j = 0; j < 16; ++j) v[j] = __uint_as_float(r[j]);
-          epilogue_store16(p, row, col0, v, cur);
-        }
-      }
+      uint8_t* st = epi_stage + (warp - 2) * EPI_STAGE_BYTES;
+      if (p.out_f32) epilogue_tile_f32<BN2>(p, bias, taddr0, st, row0, nb_ * BN2, half, lane, nullptr);
+      else epilogue_tile_bf16<BN2>(p, bias, taddr0, st, row0, nb_ * BN2, half, lane);
       tc_fence_before();
       __syncwarp();
       if (lane == 0) mbar_arrive_cluster(mapa_rank(smem_u32(&tempty_bar[acc]), 0));
@@ -849,7 +1021,8 @@ int sm_count() {
 template <int BN, int STAGES>
 int launch(const CUtensorMap& tmA, const CUtensorMap& tmB, GemmParams& p, long long ws_bytes, int ws_tiles_cap,
            cudaStream_t stream) {
-  constexpr size_t smem = (size_t)STAGES * (BM * BK * 2 + BN * BK * 2) + 1024 /*align*/ + 256 /*barriers*/;
+  constexpr size_t smem = (size_t)STAGES * (BM * BK * 2 + BN * BK * 2) + EPI_WARPS * EPI_STAGE_BYTES + 1024 /*align*/ + 256 /*barriers*/;
+  static_assert(smem <= 232448, "shared memory budget of one CTA");
   static bool configured = false;
   if (!configured) {
     NB_CUDA(cudaFuncSetAttribute(gemm_bf16_kernel<BN, STAGES>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
@@ -888,7 +1061,7 @@ int launch(const CUtensorMap& tmA, const CUtensorMap& tmB, GemmParams& p, long l
 }
 
 int launch_two_cta(const CUtensorMap& tmA, const CUtensorMap& tmB, GemmParams& p, cudaStream_t stream) {
-  constexpr size_t smem = (size_t)STAGES2 * (BM * BK * 2 + (BN2 / 2) * BK * 2) + 1024 /*align*/ + 256 /*barriers*/;
+  constexpr size_t smem = (size_t)STAGES2 * (BM * BK * 2 + (BN2 / 2) * BK * 2) + EPI_WARPS * EPI_STAGE_BYTES + 1024 /*align*/ + 256 /*barriers*/;
   static_assert(smem <= 232448, "shared memory budget of one CTA");
   static bool configured = false;
   if (!configured) {

@@ -1,0 +1,49 @@
+"""The staged GEMM epilogue at the edges of its column groups and row quarters, against fp64 on the same bf16 operands."""
+import pytest
+import torch
+
+pytestmark = pytest.mark.gpu
+
+ACTS = {None: lambda x: x, "relu": torch.relu, "gelu": lambda x: torch.nn.functional.gelu(x, approximate="tanh")}
+
+
+@pytest.mark.parametrize("m,n", [(1, 8), (33, 24), (127, 40), (129, 64), (130, 72), (255, 136), (300, 200), (513, 264), (700, 328)])
+@pytest.mark.parametrize("form", ["bias", "gelu", "residual", "f32", "accumulate", "pitch"])
+@pytest.mark.parametrize("tiles", [1, 2])
+def test_epilogue_edges(m, n, form, tiles):
+    from noeira_b200 import ops
+    from noeira_b200.ops.gemm import set_two_cta_mode
+    g = torch.Generator(device="cuda").manual_seed(m * 1000 + n)
+    k = 192
+    a = torch.randn(m, k, device="cuda", generator=g).bfloat16()
+    b = torch.randn(k, n, device="cuda", generator=g).bfloat16()
+    bias = torch.randn(n, device="cuda", generator=g)
+    res = torch.randn(m, n, device="cuda", generator=g).bfloat16()
+    exact = a.double() @ b.double()
+    kw, out = {}, None
+    if form in ("bias", "gelu"):
+        act = "gelu" if form == "gelu" else None
+        kw, exact = dict(bias=bias, act=act), ACTS[act](exact + bias.double())
+    elif form == "residual":
+        kw, exact = dict(bias=bias, residual=res), exact + bias.double() + res.double()
+    elif form == "f32":
+        kw, exact = dict(bias=bias, out_dtype=torch.float32), exact + bias.double()
+    elif form == "accumulate":
+        out = torch.randn(m, n, device="cuda", generator=g)
+        exact = exact + out.double()
+        kw = dict(out=out, accumulate=True)
+    else:                                                  # a row pitch without 16-byte rows: scalar copies, neighbours untouched
+        buf = torch.full((m, n + 3), 7.0, device="cuda", dtype=torch.bfloat16)
+        kw = dict(out=buf[:, :n])
+    old = set_two_cta_mode(tiles)
+    try:
+        y = ops.gemm(a, b, b_mn=True, **kw)
+    finally:
+        set_two_cta_mode(old)
+    # one rounding of the result to its type; the 192 fp32 products and additions; GELU through the 2^-11 hardware tanh
+    eps = 2.0 ** -8 if y.dtype == torch.bfloat16 else 0.0
+    err = (y.double() - exact).abs()
+    bound = eps * exact.abs() + 192 * 2.0 ** -23 * k ** 0.5 * 4 + (2.0 ** -9 * exact.abs() + 2e-3 if form == "gelu" else 0.0)
+    assert bool((err <= bound).all()), float((err - bound).max())
+    if form == "pitch":
+        assert bool((buf[:, n:] == 7.0).all())

@@ -46,6 +46,36 @@ fa_delta_kernel(const __nv_bfloat16* __restrict__ O, const __nv_bfloat16* __rest
   if (lane == 0) delta[((long long)b * Hq + h) * Sq + q] = acc;
 }
 
+// The same with 16-byte loads, HD / 8 lanes per row: bound by DRAM bytes (16448 x 16 x 128: 135 MB), 63 us -> 32.
+template <int HD>
+__global__ void __launch_bounds__(256)
+fa_delta_vec_kernel(const __nv_bfloat16* __restrict__ O, const __nv_bfloat16* __restrict__ dO, float* __restrict__ delta,
+                    int B, int Sq, int Hq, long long o_ss, long long do_ss) {
+  constexpr int L = HD / 8;
+  const long long row = ((long long)blockIdx.x * 256 + threadIdx.x) / L;
+  const int l = threadIdx.x % L;
+  const bool live = row < (long long)B * Sq * Hq;
+  int h = 0;
+  long long bq = 0;
+  float acc = 0.f;
+  if (live) {
+    bq = row / Hq;
+    h = (int)(row - bq * Hq);
+    const uint4 a = __ldg(reinterpret_cast<const uint4*>(O + bq * o_ss + (long long)h * HD) + l);
+    const uint4 c = __ldg(reinterpret_cast<const uint4*>(dO + bq * do_ss + (long long)h * HD) + l);
+    const __nv_bfloat162* ah = reinterpret_cast<const __nv_bfloat162*>(&a);
+    const __nv_bfloat162* ch = reinterpret_cast<const __nv_bfloat162*>(&c);
+#pragma unroll
+    for (int k = 0; k < 4; ++k) acc += __low2float(ah[k]) * __low2float(ch[k]) + __high2float(ah[k]) * __high2float(ch[k]);
+  }
+#pragma unroll
+  for (int o = L / 2; o > 0; o >>= 1) acc += __shfl_xor_sync(0xffffffffu, acc, o);
+  if (live && l == 0) {
+    const long long b = bq / Sq;
+    delta[(b * Hq + h) * Sq + (bq - b * Sq)] = acc;
+  }
+}
+
 // Two threads per query row (column halves) turn one S / dP tile pair into bf16 P and dS tiles in swizzled
 // shared memory.  sP may be null (dq kernel needs dS only).
 __device__ __forceinline__ void softmax_bwd_tile(const FaParams& p, uint32_t s_addr, uint32_t dp_addr, int q, int k0,
@@ -544,8 +574,16 @@ int nb_flash_attn_bwd(const void* Q, const void* K, const void* V, const void* O
   if (((dq_ss | dk_ss | dv_ss) * 2) % 16 != 0) return NB_ERR_UNALIGNED;
   cudaStream_t s = (cudaStream_t)stream;
   const long long rows = (long long)B * Sq * Hq;
-  fa_delta_kernel<<<(unsigned)ceil_div_ll(rows, 8), 256, 0, s>>>((const __nv_bfloat16*)O, (const __nv_bfloat16*)dO, delta,
-                                                                 B, Sq, Hq, HD, o_ss, do_ss);
+  if (o_ss % 8 == 0 && do_ss % 8 == 0 && ((reinterpret_cast<uintptr_t>(O) | reinterpret_cast<uintptr_t>(dO)) & 15) == 0) {
+    const unsigned blocks = (unsigned)ceil_div_ll(rows, 256 / (HD / 8));
+    if (HD == 64)
+      fa_delta_vec_kernel<64><<<blocks, 256, 0, s>>>((const __nv_bfloat16*)O, (const __nv_bfloat16*)dO, delta, B, Sq, Hq, o_ss, do_ss);
+    else
+      fa_delta_vec_kernel<128><<<blocks, 256, 0, s>>>((const __nv_bfloat16*)O, (const __nv_bfloat16*)dO, delta, B, Sq, Hq, o_ss, do_ss);
+  } else {
+    fa_delta_kernel<<<(unsigned)ceil_div_ll(rows, 8), 256, 0, s>>>((const __nv_bfloat16*)O, (const __nv_bfloat16*)dO, delta,
+                                                                   B, Sq, Hq, HD, o_ss, do_ss);
+  }
   NB_LAUNCH_CHECK();
   CUtensorMap tq, tk, tv, tdo;
   int rc = make_tmap_bshd(&tq, Q, B, Sq, Hq, HD, q_sb, q_ss, q_sh, BQ);

@@ -107,6 +107,136 @@ norm_fwd_kernel(const __nv_bfloat16* __restrict__ x, int ldx, const float* __res
   for (int v = lane + NV * 32; v < nvec; v += 32) emit(v, *reinterpret_cast<const uint4*>(xr + v * 8));
 }
 
+// dx, dgamma and dbeta in one pass for D <= 2048: a warp keeps a row of x and dy packed in registers between the two sums and
+// dx, and carries its columns' parameter gradients in registers down all its rows (blocks walk the rows), so x and dy are read
+// once.  Bound by DRAM bytes; 8 or 16 warps with 2 x NV 16-byte loads each keep enough in flight.  The separate kernels below
+// read x and dy four times (twice for dx, once for the parameters, which finished with one thread per column): 16448 x 2048
+// RMS 106 + 36 + 7 us, here 56 + 4.
+// Threads of a block (one per SM): more warps where a row takes few registers.
+__host__ __device__ constexpr int norm_bwd_threads(int nv) { return nv >= 8 ? 256 : 512; }
+template <bool RMS, int NV>
+__global__ void __launch_bounds__(norm_bwd_threads(NV), 1)
+norm_bwd_fused_kernel(const __nv_bfloat16* __restrict__ x, int ldx, const __nv_bfloat16* __restrict__ dy, int lddy,
+                      const float* __restrict__ gamma, const float2* __restrict__ stats, __nv_bfloat16* __restrict__ dx,
+                      int lddx, float* __restrict__ pg, float* __restrict__ pb, int M, int D, int accumulate) {
+  constexpr int T = norm_bwd_threads(NV), WARPS = T / 32;
+  extern __shared__ float4 nb_sh4[];            // gamma: [2][NV * 32] float4 halves of 8 columns; later the block's sums
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, nvec = D / 8;
+  for (int i = threadIdx.x; i < 2 * nvec; i += T) {
+    const int v = i >> 1, h = i & 1;
+    float4 g = make_float4(1.f, 1.f, 1.f, 1.f);
+    if (gamma) {
+      const float* q = gamma + v * 8 + h * 4;
+      g = make_float4(q[0], q[1], q[2], q[3]);
+    }
+    nb_sh4[h * (NV * 32) + v] = g;
+  }
+  __syncthreads();
+  float ag[NV][8], ab[RMS ? 1 : NV][8];
+#pragma unroll
+  for (int k = 0; k < NV; ++k)
+#pragma unroll
+    for (int i = 0; i < 8; ++i) {
+      ag[k][i] = 0.f;
+      if (!RMS) ab[RMS ? 0 : k][i] = 0.f;
+    }
+  const float invD = 1.f / D;
+  for (int row = blockIdx.x * WARPS + warp; row < M; row += gridDim.x * WARPS) {
+    const __nv_bfloat16* xr = x + (size_t)row * ldx;
+    const __nv_bfloat16* dr = dy + (size_t)row * lddy;
+    uint4 cx[NV], cd[NV];
+#pragma unroll
+    for (int k = 0; k < NV; ++k) {
+      const int v = lane + k * 32;
+      if (v < nvec) {
+        cx[k] = __ldg(reinterpret_cast<const uint4*>(xr + v * 8));
+        cd[k] = __ldg(reinterpret_cast<const uint4*>(dr + v * 8));
+      }
+    }
+    const float2 st = stats[row];
+    float s1 = 0.f, s2 = 0.f;
+#pragma unroll
+    for (int k = 0; k < NV; ++k) {
+      const int v = lane + k * 32;
+      if (v < nvec) {
+        float a[8], g[8];
+        unpack8(cx[k], a);
+        unpack8(cd[k], g);
+        const float4 w0 = nb_sh4[v], w1 = nb_sh4[NV * 32 + v];
+        const float w[8] = {w0.x, w0.y, w0.z, w0.w, w1.x, w1.y, w1.z, w1.w};
+#pragma unroll
+        for (int i = 0; i < 8; ++i) {
+          const float xh = (a[i] - st.x) * st.y, gg = g[i] * w[i];
+          s1 += gg;
+          s2 += gg * xh;
+          ag[k][i] += g[i] * xh;
+          if (!RMS) ab[RMS ? 0 : k][i] += g[i];
+        }
+      }
+    }
+    s1 = RMS ? 0.f : warp_sum(s1) * invD;
+    s2 = warp_sum(s2) * invD;
+    if (dx) {
+      __nv_bfloat16* orow = dx + (size_t)row * lddx;
+#pragma unroll
+      for (int k = 0; k < NV; ++k) {
+        const int v = lane + k * 32;
+        if (v < nvec) {
+          float a[8], g[8], o[8];
+          unpack8(cx[k], a);
+          unpack8(cd[k], g);
+          if (accumulate) unpack8(*reinterpret_cast<const uint4*>(orow + v * 8), o);
+          const float4 w0 = nb_sh4[v], w1 = nb_sh4[NV * 32 + v];
+          const float w[8] = {w0.x, w0.y, w0.z, w0.w, w1.x, w1.y, w1.z, w1.w};
+#pragma unroll
+          for (int i = 0; i < 8; ++i) {
+            const float d = st.y * (g[i] * w[i] - s1 - (a[i] - st.x) * st.y * s2);
+            o[i] = accumulate ? o[i] + d : d;
+          }
+          *reinterpret_cast<uint4*>(orow + v * 8) = pack8(o);
+        }
+      }
+    }
+  }
+  if (!pg) return;
+  // the warps' parameter sums, halved in a fixed order: the upper half of the warps hands its sums to the lower half
+  float* sum = reinterpret_cast<float*>(nb_sh4);
+#pragma unroll
+  for (int pass = 0; pass < (RMS ? 1 : 2); ++pass) {
+    if (pass == 1 && !pb) break;
+#pragma unroll 1
+    for (int n = WARPS / 2; n > 0; n >>= 1) {
+      __syncthreads();
+#pragma unroll
+      for (int k = 0; k < NV; ++k)
+#pragma unroll
+        for (int i = 0; i < 8; ++i)
+          if (warp >= n && warp < 2 * n) sum[(warp - n) * (NV * 256) + i * (NV * 32) + lane + k * 32] = pass == 0 ? ag[k][i] : ab[RMS ? 0 : k][i];
+      __syncthreads();
+      if (warp < n) {
+#pragma unroll
+        for (int k = 0; k < NV; ++k)
+#pragma unroll
+          for (int i = 0; i < 8; ++i) {
+            float& t = pass == 0 ? ag[k][i] : ab[RMS ? 0 : k][i];
+            t += sum[warp * (NV * 256) + i * (NV * 32) + lane + k * 32];
+          }
+      }
+    }
+    if (warp == 0) {
+      float* out = (pass == 0 ? pg : pb) + (size_t)blockIdx.x * D;
+#pragma unroll
+      for (int k = 0; k < NV; ++k) {
+        const int v = lane + k * 32;
+        if (v < nvec) {
+#pragma unroll
+          for (int i = 0; i < 8; ++i) out[v * 8 + i] = pass == 0 ? ag[k][i] : ab[RMS ? 0 : k][i];
+        }
+      }
+    }
+  }
+}
+
 // dx = rstd * (g - mean(g) - xhat * mean(g * xhat)),  g = dy * gamma   (RMS: no mean(g) term)
 template <bool RMS>
 __global__ void __launch_bounds__(256)
@@ -195,15 +325,27 @@ norm_bwd_params_kernel(const __nv_bfloat16* __restrict__ x, int ldx, const __nv_
   }
 }
 
-__global__ void norm_bwd_params_finish_kernel(const float* __restrict__ pg, const float* __restrict__ pb, int D,
-                                              int split, float* __restrict__ dgamma, float* __restrict__ dbeta) {
-  const int c = blockIdx.x * blockDim.x + threadIdx.x;
-  if (c >= D) return;
+// 32 columns per block: 8 warps take every 8th partial each, then the 8 sums are added in order
+__global__ void __launch_bounds__(256)
+norm_bwd_params_finish_kernel(const float* __restrict__ pg, const float* __restrict__ pb, int D, int split,
+                              float* __restrict__ dgamma, float* __restrict__ dbeta) {
+  __shared__ float qg[8][33], qb[8][33];
+  const int l = threadIdx.x & 31, w = threadIdx.x >> 5, c = blockIdx.x * 32 + l;
   float sg = 0.f, sb = 0.f;
-  for (int k = 0; k < split; ++k) {
-    sg += pg[(size_t)k * D + c];
-    if (pb) sb += pb[(size_t)k * D + c];
+  if (c < D) {
+#pragma unroll 8
+    for (int k = w; k < split; k += 8) {
+      sg += pg[(size_t)k * D + c];
+      if (pb) sb += pb[(size_t)k * D + c];
+    }
   }
+  qg[w][l] = sg;
+  qb[w][l] = sb;
+  __syncthreads();
+  if (w != 0 || c >= D) return;
+  sg = sb = 0.f;
+#pragma unroll
+  for (int k = 0; k < 8; ++k) { sg += qg[k][l]; sb += qb[k][l]; }
   if (dgamma) dgamma[c] += sg;
   if (dbeta && pb) dbeta[c] += sb;
 }
@@ -212,9 +354,10 @@ __global__ void norm_bwd_params_finish_kernel(const float* __restrict__ pg, cons
 
 extern "C" {
 
+// number of partial sums per column = blocks of the backward: one per SM, each with at least one row per warp
 int nb_norm_split(int M) {
-  int s = M / 64;
-  return s < 1 ? 1 : (s > 128 ? 128 : s);
+  const int s = ceil_div(M, 8);
+  return s < 1 ? 1 : (s > 148 ? 148 : s);
 }
 
 // rms != 0 → RMSNorm.  stats: M float2 (mean, rstd) kept for the backward.
@@ -250,6 +393,34 @@ int nb_norm_bwd(const void* x, int ldx, const void* dy, int lddy, const float* g
   if (D % 8 || ldx % 8 || lddy % 8 || lddx % 8) return NB_ERR_UNALIGNED;
   cudaStream_t s = (cudaStream_t)stream;
   dim3 grid(ceil_div(M, 8));
+  if (D <= MAXV * 256 && (dx || dgamma)) {
+    const int split = nb_norm_split(M), need = ceil_div(D, 256);
+    float* pg = dgamma ? partials : nullptr;
+    float* pb = (rms || !dbeta || !dgamma) ? nullptr : partials + (size_t)split * D;
+#define NB_NORM_BWD(R, NVV)                                                                                                   \
+  norm_bwd_fused_kernel<R, NVV><<<split, norm_bwd_threads(NVV), norm_bwd_threads(NVV) / 64 * NVV * 256 * sizeof(float), s>>>(       \
+      (const __nv_bfloat16*)x, ldx, (const __nv_bfloat16*)dy, lddy, gamma, (const float2*)stats, (__nv_bfloat16*)dx, lddx, pg, \
+      pb, M, D, accumulate_dx)
+    if (rms) {
+      if (need <= 1) NB_NORM_BWD(true, 1);
+      else if (need <= 2) NB_NORM_BWD(true, 2);
+      else if (need <= 4) NB_NORM_BWD(true, 4);
+      else NB_NORM_BWD(true, 8);
+    } else {
+      if (need <= 1) NB_NORM_BWD(false, 1);
+      else if (need <= 2) NB_NORM_BWD(false, 2);
+      else if (need <= 4) NB_NORM_BWD(false, 4);
+      else NB_NORM_BWD(false, 8);
+    }
+#undef NB_NORM_BWD
+    NB_LAUNCH_CHECK();
+    if (dgamma) {
+      norm_bwd_params_finish_kernel<<<ceil_div(D, 32), 256, 0, s>>>(pg, pb, D, split, dgamma, dbeta);
+      NB_LAUNCH_CHECK();
+    }
+    return NB_OK;
+  }
+  // wider rows: one kernel for dx, one for the parameter gradients
   if (dx) {
     if (rms)
       norm_bwd_dx_kernel<true><<<grid, 256, 0, s>>>((const __nv_bfloat16*)x, ldx, (const __nv_bfloat16*)dy, lddy, gamma,
@@ -268,7 +439,7 @@ int nb_norm_bwd(const void* x, int ldx, const void* dy, int lddy, const float* g
     norm_bwd_params_kernel<<<dim3(ceil_div(D, 256), ceil_div(M, rows)), 256, 0, s>>>(
         (const __nv_bfloat16*)x, ldx, (const __nv_bfloat16*)dy, lddy, (const float2*)stats, pg, pb, M, D, rows);
     NB_LAUNCH_CHECK();
-    norm_bwd_params_finish_kernel<<<ceil_div(D, 128), 128, 0, s>>>(pg, pb, D, ceil_div(M, rows), dgamma, dbeta);
+    norm_bwd_params_finish_kernel<<<ceil_div(D, 32), 256, 0, s>>>(pg, pb, D, ceil_div(M, rows), dgamma, dbeta);
     NB_LAUNCH_CHECK();
   }
   return NB_OK;

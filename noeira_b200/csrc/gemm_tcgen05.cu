@@ -5,8 +5,8 @@
 //     64-wide k-block; tcgen05.commit releases the stage / publishes the accumulator;
 //   * persistent CTAs (one per SM) walk the tile list; two TMEM accumulators let the epilogue
 //     of tile i overlap the main loop of tile i+1;
-//   * warp roles (320 threads): warp 0 = TMA producer, warp 1 = MMA issuer + TMEM owner,
-//     warps 2..9 = epilogue (TMEM quarter = warp_id % 4, two warps per quarter);
+//   * warp roles (352 threads): warp 0 = TMA producer of A, warp 1 = MMA issuer + TMEM owner, warp 2 = TMA producer of B,
+//     warps 3..10 = epilogue (TMEM quarter = warp_id % 4, two warps per quarter);
 //   * both operands may be K-major ([rows, K] row-major) or MN-major ([K, rows] row-major), so
 //     forward (x·W, W stored [IN, OUT]), dgrad (dy·Wᵀ) and wgrad (xᵀ·dy) all run from the
 //     natural layouts without a transpose pass;
@@ -34,7 +34,8 @@ constexpr int UMMA_K = 16;
 // epilogue of a 256 x 256 tile (bias, GELU, residual, bf16 store) took longer than the twelve k-blocks of K = 768, and the
 // tensor core waited for a free accumulator: 24576 x 3072 x 768 with GELU took 240 us, 176 us with eight.
 constexpr int EPI_WARPS = 8;
-constexpr int NUM_THREADS = 64 + 32 * EPI_WARPS;
+constexpr int NUM_THREADS = 96 + 32 * EPI_WARPS;     // A loads, MMA, B loads, epilogue
+constexpr int NUM_THREADS2 = 64 + 32 * EPI_WARPS;    // CTA pairs: loads, MMA, epilogue
 
 struct GemmParams {
   int M, N, K;
@@ -45,6 +46,7 @@ struct GemmParams {
   int out_f32, accumulate, act, dact;
   int tiles_m, tiles_n, num_kb;
   int splits, kb_per_split;  // split-K: work item = (tile, split); partial tiles meet in `ws`
+  int tile_rows;             // rows of a tile: BM, 2 BM for CTA pairs
   float alpha;
   float* ws;                 // splits>1: fp32 partial tiles, [tile][split][BM*BN]
   unsigned int* tile_ctr;    // splits>1: one arrival counter per tile (zero between launches)
@@ -87,8 +89,9 @@ __device__ __forceinline__ void act_apply16(int act, float (&v)[16]) {
     case NB_ACT_GELU:
 #pragma unroll
       for (int j = 0; j < 16; ++j) {
-        const float x = v[j];
-        v[j] = 0.5f * x * (1.f + tanh_fast(0.7978845608028654f * (x + 0.044715f * x * x * x)));
+        // 0.5 x (1 + tanh(c (x + 0.044715 x^3))) in five multiply-adds around the tanh
+        const float x = v[j], h = 0.5f * x;
+        v[j] = fmaf(h, tanh_fast(x * fmaf(0.7978845608028654f * 0.044715f, x * x, 0.7978845608028654f)), h);
       }
       break;
     case NB_ACT_SILU:
@@ -173,8 +176,21 @@ __device__ __forceinline__ void epilogue_prefetch16(const GemmParams& p, int row
   }
 }
 
+// What a tile's epilogue does is part of the kernel: the frequent forms have instances of their own.  With the tests for
+// bias, activation and saved tensor inside the loop over 16-column chunks every chunk jumped across the whole switch, and a
+// chunk without any of them took 530 clocks, most of them instruction fetch; it takes 165 now.  (All forms side by side in
+// one kernel spilled 4 KB of registers.)  The bias is a run-time test everywhere: one jump over 16 shuffles.
+enum EpiMode { EPI_PLAIN, EPI_RELU, EPI_GELU, EPI_ADD, EPI_BF16, EPI_F32, EPI_F32_ANY, EPI_MODES };   // EPI_BF16, EPI_F32_ANY: the rest
+__host__ inline EpiMode epi_mode(const GemmParams& p, bool split) {
+  if (split) return EPI_F32;                                                   // raw partial tiles
+  if (p.out_f32) return (!p.bias && !p.act && !p.dact) ? EPI_F32 : EPI_F32_ANY;
+  if (!p.dact) return !p.act ? EPI_PLAIN : (p.act == NB_ACT_RELU ? EPI_RELU : (p.act == NB_ACT_GELU ? EPI_GELU : EPI_BF16));
+  return (!p.act && p.dact == NB_AUX_ADD) ? EPI_ADD : EPI_BF16;
+}
+
 // alpha, bias and activation of 16 consecutive columns; `sv`: the 16 values of the saved / residual tensor when dact is set.
 // The bias comes from the lanes that hold it (see load_bias): lane b0 + j has columns 4j .. 4j + 3 of the chunk.
+template <int MODE>
 __device__ __forceinline__ void epilogue_math16(const GemmParams& p, const float4& bias, int b0, float (&v)[16], const float (&sv)[16]) {
 #pragma unroll
   for (int j = 0; j < 16; ++j) v[j] *= p.alpha;
@@ -187,8 +203,13 @@ __device__ __forceinline__ void epilogue_math16(const GemmParams& p, const float
       v[4 * j + 3] += __shfl_sync(0xffffffffu, bias.w, b0 + j);
     }
   }
-  if (p.act) act_apply16(p.act, v);
-  if (p.dact) dact_apply16(p.dact, v, sv);
+  if (MODE == EPI_RELU) act_apply16(NB_ACT_RELU, v);
+  if (MODE == EPI_GELU) act_apply16(NB_ACT_GELU, v);
+  if (MODE == EPI_ADD) dact_apply16(NB_AUX_ADD, v, sv);
+  if (MODE == EPI_BF16 || MODE == EPI_F32_ANY) {
+    if (p.act) act_apply16(p.act, v);
+    if (p.dact) dact_apply16(p.dact, v, sv);
+  }
 }
 // The bias of a warp's column groups (`half`, `half` + 2, ... of G columns each; at most 128 columns), four per lane, fetched
 // while the accumulator is still being computed.  Loaded inside the chunk loop it cost an L2 round trip per 16 columns (most
@@ -293,7 +314,8 @@ __device__ __forceinline__ void epilogue_store16(const GemmParams& p, int row, i
 //
 // Tensor memory hands every lane a whole row, and a store straight from there touches 32 rows with 16 bytes each: 32 L2
 // requests per instruction, which made GEMMs with K <= 1024 epilogue-bound (24576 x 2304 x 768 with bias: 142 us with direct
-// stores from four warps, 105 us from eight, 101 us staged, 82 us with the bias fetched ahead, see load_bias).  So a group goes through 4 KB of shared memory per warp: the lane that
+// stores from four warps, 105 us from eight, 101 us staged, 82 us with the bias fetched ahead, see load_bias,
+// and 71 with a kernel per epilogue form, see EpiMode).  So a group goes through 4 KB of shared memory per warp: the lane that
 // owns the row does the arithmetic and writes its packed row (16-byte chunks XOR-swizzled, no bank conflicts), then the warp
 // copies the group out with whole 64- or 128-byte row segments per request.  The saved / residual tensor comes in the same
 // way in front of the arithmetic, the old fp32 output is added during the copy.
@@ -307,8 +329,8 @@ __device__ __forceinline__ int epi_off(int r, int ch) {
 
 template <int BN>
 __host__ __device__ constexpr int epi_group() { return BN >= 128 ? 64 : 32; }   // columns per group, bf16 output
-template <int BN>
-__device__ __forceinline__ void epilogue_tile_bf16(const GemmParams& p, const float4& bias, uint32_t taddr, uint8_t* st, int row0,
+template <int BN, int MODE>
+__device__ __forceinline__ void epilogue_groups_bf16(const GemmParams& p, const float4& bias, uint32_t taddr, uint8_t* st, int row0,
                                                    int n0, int half, int lane) {
   constexpr int G = epi_group<BN>(), CPR = G / 8, NV = CPR;   // columns per group; 16-byte vectors per lane and group
   constexpr int NC = (BN < G ? BN : G) / 16;                      // 16-column chunks per group
@@ -326,41 +348,51 @@ __device__ __forceinline__ void epilogue_tile_bf16(const GemmParams& p, const fl
         if (vec_a && col + 8 <= p.N) {
           ax[i] = __ldg(reinterpret_cast<const uint4*>(a));
         } else {
-          __nv_bfloat16 e[8];
-#pragma unroll
-          for (int j = 0; j < 8; ++j) e[j] = col + j < p.N ? a[j] : __float2bfloat16(0.f);
-          ax[i] = *reinterpret_cast<const uint4*>(e);
+          auto at = [&](int j) { return col + j < p.N ? (uint32_t)__bfloat16_as_ushort(a[j]) : 0u; };
+          ax[i] = make_uint4(at(0) | at(1) << 16, at(2) | at(3) << 16, at(4) | at(5) << 16, at(6) | at(7) << 16);
         }
       }
       a += (size_t)RS * p.ld_aux;
     }
   };
-  if (p.dact && half * G < BN && n0 + half * G < p.N) load_aux(half * G);
+  const bool with_aux = MODE == EPI_ADD || (MODE == EPI_BF16 && p.dact != 0);
+  if (with_aux && half * G < BN && n0 + half * G < p.N) load_aux(half * G);
 #pragma unroll 1
   for (int c = half * G; c < BN && n0 + c < p.N; c += 2 * G) {
-    if (p.dact) {
+    if (with_aux) {
 #pragma unroll
       for (int i = 0; i < NV; ++i) *reinterpret_cast<uint4*>(st + epi_off<CPR>(rr0 + i * RS, ch)) = ax[i];
       __syncwarp();
       if (c + 2 * G < BN && n0 + c + 2 * G < p.N) load_aux(c + 2 * G);
     }
-#pragma unroll 1
-    for (int k = 0; k < NC; ++k) {
-      uint32_t r[16];
-      tmem_ld_32x32b_x16(taddr + (uint32_t)(c + 16 * k), r);
-      tmem_ld_wait();
+    auto chunk = [&](int k, const uint32_t* r) {
       float v[16], sv[16];
 #pragma unroll
       for (int j = 0; j < 16; ++j) v[j] = __uint_as_float(r[j]);
       uint8_t* s0 = st + epi_off<CPR>(lane, 2 * k);
       uint8_t* s1 = st + epi_off<CPR>(lane, 2 * k + 1);
-      if (p.dact) {
+      if (with_aux) {
         const uint4 w[2] = {*reinterpret_cast<const uint4*>(s0), *reinterpret_cast<const uint4*>(s1)};
         unpack16(w, sv);
       }
-      epilogue_math16(p, bias, ((c / (2 * G)) * G + 16 * k) >> 2, v, sv);
+      epilogue_math16<MODE>(p, bias, ((c / (2 * G)) * G + 16 * k) >> 2, v, sv);
       *reinterpret_cast<uint4*>(s0) = pack8f(v);
       *reinterpret_cast<uint4*>(s1) = pack8f(v + 8);
+    };
+    if (NC == 1) {
+      uint32_t r[16];
+      tmem_ld_32x32b_x16(taddr + (uint32_t)c, r);
+      tmem_ld_wait();
+      chunk(0, r);
+    } else {
+#pragma unroll 1
+      for (int k = 0; k < NC; k += 2) {       // two chunks per tensor-memory load
+        uint32_t r[32];
+        tmem_ld_32x32b_x32(taddr + (uint32_t)(c + 16 * k), r);
+        tmem_ld_wait();
+        chunk(k, r);
+        chunk(k + 1, r + 16);
+      }
     }
     __syncwarp();
     const int col = n0 + c + ch * 8;
@@ -388,35 +420,46 @@ __device__ __forceinline__ void epilogue_tile_bf16(const GemmParams& p, const fl
 }
 
 // fp32 output, or (split) the raw fp32 partial tile of a split-K item at `part` (row pitch BN)
-template <int BN>
-__device__ __forceinline__ void epilogue_tile_f32(const GemmParams& p, const float4& bias, uint32_t taddr, uint8_t* st, int row0,
+template <int BN, int MODE>
+__device__ __forceinline__ void epilogue_groups_f32(const GemmParams& p, const float4& bias, uint32_t taddr, uint8_t* st, int row0,
                                                   int n0, int half, int lane, float* part) {
   constexpr int G = 32;
   constexpr int NC = (BN < G ? BN : G) / 16;
   const bool vec_d = p.ldd % 4 == 0;
 #pragma unroll 1
   for (int c = half * G; c < BN && n0 + c < p.N; c += 2 * G) {
-#pragma unroll 1
-    for (int k = 0; k < NC; ++k) {
-      uint32_t r[16];
-      tmem_ld_32x32b_x16(taddr + (uint32_t)(c + 16 * k), r);
-      tmem_ld_wait();
+    auto chunk = [&](int k, const uint32_t* r) {
       float v[16];
 #pragma unroll
       for (int j = 0; j < 16; ++j) v[j] = __uint_as_float(r[j]);
       const int col0 = n0 + c + 16 * k;
-      if (!part) {
+      if (MODE == EPI_F32_ANY) {
         float sv[16];
         if (p.dact) {
           const __nv_bfloat16* ax = p.aux + (size_t)(row0 + lane) * p.ld_aux + col0;
 #pragma unroll
           for (int j = 0; j < 16; ++j) sv[j] = (row0 + lane < p.M && col0 + j < p.N) ? __bfloat162float(ax[j]) : 0.f;
         }
-        epilogue_math16(p, bias, ((c / (2 * G)) * G + 16 * k) >> 2, v, sv);
+        epilogue_math16<MODE>(p, bias, ((c / (2 * G)) * G + 16 * k) >> 2, v, sv);
+      } else if (!part) {
+#pragma unroll
+        for (int j = 0; j < 16; ++j) v[j] *= p.alpha;
       }
 #pragma unroll
       for (int j = 0; j < 4; ++j)
         *reinterpret_cast<float4*>(st + epi_off<8>(lane, 4 * k + j)) = make_float4(v[4 * j], v[4 * j + 1], v[4 * j + 2], v[4 * j + 3]);
+    };
+    if (NC == 1) {
+      uint32_t r[16];
+      tmem_ld_32x32b_x16(taddr + (uint32_t)c, r);
+      tmem_ld_wait();
+      chunk(0, r);
+    } else {
+      uint32_t r[32];
+      tmem_ld_32x32b_x32(taddr + (uint32_t)c, r);
+      tmem_ld_wait();
+      chunk(0, r);
+      chunk(1, r + 16);
     }
     __syncwarp();
     const int rr0 = lane >> 3, ch = lane & 7, col = n0 + c + ch * 4;
@@ -459,6 +502,36 @@ __device__ __forceinline__ void epilogue_tile_f32(const GemmParams& p, const flo
   }
 }
 
+// Bounded wait of a pipeline role.  The common case is one test of the barrier; the abort flag of the CTA is looked at only
+// while the barrier is not there yet.
+__device__ __forceinline__ bool wait_or_abort(uint64_t* bar, uint32_t parity, volatile uint32_t* abort_flag, unsigned int* status,
+                                              unsigned int where) {
+  if (mbar_try_wait(bar, parity)) return true;
+  for (uint32_t it = 0; it < NB_SPIN_LIMIT; ++it) {
+    if (mbar_try_wait(bar, parity)) return true;
+    if ((it & 63u) == 0u && *abort_flag) return false;
+  }
+  report(status, NB_ST_MBAR_TIMEOUT, where, parity);
+  return false;
+}
+
+// The four instructions of one k-block.  `ad` / `bd` are complete descriptors of the stage's operands, `astep` / `bstep` the
+// advance per instruction in descriptor units (16 bytes).  Nothing but additions stands between two instructions: with the
+// descriptors built from the operand majors in front of each one, the issuing thread needed 880 clocks per k-block, three to
+// six times what the tensor core needs for it (M = 128: 512 clocks at 256 columns, 128 at 64), and every one-CTA tile ran at
+// 416 ns per k-block whatever its width; 190 to 280 ns now.
+template <bool TF32>
+__device__ __forceinline__ void mma_kblock(uint32_t d_tmem, uint64_t ad, uint64_t bd, uint32_t astep, uint32_t bstep, uint32_t idesc,
+                                           uint32_t accumulate) {
+#pragma unroll
+  for (int k = 0; k < BK / UMMA_K; ++k) {
+    if (TF32) umma_tf32(d_tmem, ad, bd, idesc, k == 0 ? accumulate : 1u);
+    else umma_f16(d_tmem, ad, bd, idesc, k == 0 ? accumulate : 1u);
+    ad += astep;
+    bd += bstep;
+  }
+}
+
 __device__ __forceinline__ void tile_coords(int tile, int tiles_m, int tiles_n, int& mb, int& nb_) {
   constexpr int GM = 8;
   const int per_group = GM * tiles_n;
@@ -470,7 +543,7 @@ __device__ __forceinline__ void tile_coords(int tile, int tiles_m, int tiles_n, 
   nb_ = in_group / gsz;
 }
 
-template <int BN, int STAGES>
+template <int BN, int STAGES, int MODE>
 __global__ void __launch_bounds__(NUM_THREADS, 1)
 gemm_bf16_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmB,
                  const GemmParams p) {
@@ -488,7 +561,6 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
   uint64_t* tempty_bar = tfull_bar + 2;
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(tempty_bar + 2);
   volatile uint32_t* abort_flag = tmem_slot + 1;
-  volatile uint32_t* ticket_slot = tmem_slot + 2;
 
   const int warp = threadIdx.x >> 5;
   const int lane = threadIdx.x & 31;
@@ -496,7 +568,7 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
 
   if (threadIdx.x == 0) {
     for (int s = 0; s < STAGES; ++s) {
-      mbar_init(&full_bar[s], 1);
+      mbar_init(&full_bar[s], 2);   // both producers announce their bytes
       mbar_init(&empty_bar[s], 1);
     }
     for (int a = 0; a < 2; ++a) {
@@ -517,8 +589,11 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
   tc_fence_after();
   const uint32_t tmem_base = *tmem_slot;
 
-  if (warp == 0) {
-    // ------------------------------------------------------------------ TMA producer
+  if (warp == 0 || warp == 2) {
+    // ------------------------------------------------------------------ TMA producers
+    // One thread for A, one for B: a thread needs about 100 ns per k-block and 50 ns per copy, which for one thread with the
+    // two to six copies of a stage is more than the tensor core needs for it (M = N = 128: 209 to 317 ns per k-block with
+    // one producer thread, 191 to 238 with two).
     if (elect_one()) {
       int stage = 0;
       uint32_t phase = 0;
@@ -532,11 +607,18 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
         tile_coords(tile, p.tiles_m, p.tiles_n, mb, nb_);
         const int kb0 = split * p.kb_per_split, kb1 = min(p.num_kb, kb0 + p.kb_per_split);
         for (int kb = kb0; kb < kb1; ++kb) {
-          if (*abort_flag || !mbar_wait(&empty_bar[stage], phase ^ 1u, p.status, 1)) { ok = false; *abort_flag = 1; break; }
+          if (!wait_or_abort(&empty_bar[stage], phase ^ 1u, abort_flag, p.status, 1)) { ok = false; *abort_flag = 1; break; }
           uint8_t* sa = smem + stage * STAGE_BYTES;
           uint8_t* sb = sa + A_BYTES;
-          mbar_expect_tx(&full_bar[stage], STAGE_BYTES);
-          if (p.conv == 2) {
+          mbar_expect_tx(&full_bar[stage], warp == 0 ? A_BYTES : B_BYTES);
+          if (warp == 2) {
+            if (!p.b_mn) {
+              tma_load_2d(sb, &tmB, &full_bar[stage], kb * bk, nb_ * BN);
+            } else {
+              for (int h = 0; h < (BN + chunk - 1) / chunk; ++h)
+                tma_load_2d(sb + h * (bk * 128), &tmB, &full_bar[stage], nb_ * BN + h * chunk, kb * bk);
+            }
+          } else if (p.conv == 2) {
             // rows of the tile = 2 chunks of 64 channels of one filter tap each; k-block kb = 64 output pixels as runs of
             // bw consecutive pixels of one output row.  A chunk past the last tap and pixels past the last image read the
             // zero fill (image index out of range), so the byte count of the stage stays the same.
@@ -573,12 +655,6 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
             for (int h = 0; h < BM / chunk; ++h)
               tma_load_2d(sa + h * (bk * 128), &tmA, &full_bar[stage], mb * BM + h * chunk, kb * bk);
           }
-          if (!p.b_mn) {
-            tma_load_2d(sb, &tmB, &full_bar[stage], kb * bk, nb_ * BN);
-          } else {
-            for (int h = 0; h < (BN + chunk - 1) / chunk; ++h)
-              tma_load_2d(sb + h * (bk * 128), &tmB, &full_bar[stage], nb_ * BN + h * chunk, kb * bk);
-          }
           if (++stage == STAGES) { stage = 0; phase ^= 1u; }
         }
       }
@@ -588,38 +664,35 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
     if (elect_one()) {
       const uint32_t idesc = make_idesc(p.tf32 ? 2u : 1u, BM, BN, (uint32_t)p.a_mn, (uint32_t)p.b_mn);
       // one instruction consumes 32 bytes of K: 16 bf16 or 8 tf32.  K-major: 32 bytes further inside the swizzle row;
-      // MN-major: that many k-rows of 128 bytes further, chunks of MN one k-block of rows apart
-      // an MN-major TF32 operand is in the 32-byte-atom form of the 128-byte swizzle (descriptor layout 1): its pattern
-      // repeats every 4 k-rows, so the stride between row groups is 512 bytes instead of 1024
-      const uint32_t kadv_mn = p.tf32 ? 8u * 128u : 16u * 128u, lbo_mn = p.tf32 ? 32u * 128u : 64u * 128u;
-      const uint32_t sbo_mn = p.tf32 ? 512u : 1024u, lay_mn = p.tf32 ? 1u : 2u;
+      // MN-major: that many k-rows of 128 bytes further, chunks of MN one k-block of rows apart.
+      // An MN-major TF32 operand is in the 32-byte-atom form of the 128-byte swizzle (descriptor layout 1): its pattern
+      // repeats every 4 k-rows, so the stride between row groups is 512 bytes instead of 1024.
       const bool tf32 = p.tf32 != 0;
+      const uint32_t kadv_mn = tf32 ? 8u * 128u : 16u * 128u, lbo_mn = tf32 ? 32u * 128u : 64u * 128u;
+      const uint32_t sbo_mn = tf32 ? 512u : 1024u, lay_mn = tf32 ? 1u : 2u;
+      const uint32_t s0 = smem_u32(smem);
+      const uint64_t ad0 = p.a_mn ? make_smem_desc(s0, lbo_mn, sbo_mn, lay_mn) : make_smem_desc(s0, 16, 1024, 2);
+      const uint64_t bd0 = p.b_mn ? make_smem_desc(s0 + A_BYTES, lbo_mn, sbo_mn, lay_mn) : make_smem_desc(s0 + A_BYTES, 16, 1024, 2);
+      const uint32_t astep = (p.a_mn ? kadv_mn : UMMA_K * 2) >> 4, bstep = (p.b_mn ? kadv_mn : UMMA_K * 2) >> 4;
       int stage = 0;
       uint32_t phase = 0;
       int acc = 0;
       uint32_t acc_phase = 0;
       bool ok = true;
       for (int item = blockIdx.x; item < num_items && ok; item += gridDim.x) {
-        if (*abort_flag || !mbar_wait(&tempty_bar[acc], acc_phase ^ 1u, p.status, 2)) { ok = false; *abort_flag = 1; break; }
+        if (!wait_or_abort(&tempty_bar[acc], acc_phase ^ 1u, abort_flag, p.status, 2)) { ok = false; *abort_flag = 1; break; }
         tc_fence_after();
         const uint32_t d_tmem = tmem_base + (uint32_t)(acc * BN);
         const int split = item % p.splits;
         const int kb0 = split * p.kb_per_split, kb1 = min(p.num_kb, kb0 + p.kb_per_split);
+        uint32_t accumulate = 0;
         for (int kb = kb0; kb < kb1; ++kb) {
-          if (*abort_flag || !mbar_wait(&full_bar[stage], phase, p.status, 3)) { ok = false; *abort_flag = 1; break; }
+          if (!wait_or_abort(&full_bar[stage], phase, abort_flag, p.status, 3)) { ok = false; *abort_flag = 1; break; }
           tc_fence_after();
-          const uint32_t sa = smem_u32(smem + stage * STAGE_BYTES);
-          const uint32_t sb = sa + A_BYTES;
-#pragma unroll
-          for (int k = 0; k < BK / UMMA_K; ++k) {
-            // K-major: advance 32 bytes inside the 128B swizzle row; MN-major: 16 k-rows of 128 B
-            const uint64_t adesc = p.a_mn ? make_smem_desc(sa + k * kadv_mn, lbo_mn, sbo_mn, lay_mn)
-                                          : make_smem_desc(sa + k * (UMMA_K * 2), 16, 1024, 2);
-            const uint64_t bdesc = p.b_mn ? make_smem_desc(sb + k * kadv_mn, lbo_mn, sbo_mn, lay_mn)
-                                          : make_smem_desc(sb + k * (UMMA_K * 2), 16, 1024, 2);
-            if (tf32) umma_tf32(d_tmem, adesc, bdesc, idesc, ((kb - kb0) | k) != 0 ? 1u : 0u);
-            else umma_f16(d_tmem, adesc, bdesc, idesc, ((kb - kb0) | k) != 0 ? 1u : 0u);
-          }
+          const uint32_t off = (uint32_t)stage * (STAGE_BYTES >> 4);
+          if (tf32) mma_kblock<true>(d_tmem, ad0 + off, bd0 + off, astep, bstep, idesc, accumulate);
+          else mma_kblock<false>(d_tmem, ad0 + off, bd0 + off, astep, bstep, idesc, accumulate);
+          accumulate = 1;
           umma_commit(&empty_bar[stage]);
           if (++stage == STAGES) { stage = 0; phase ^= 1u; }
         }
@@ -629,8 +702,8 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
       }
     }
   } else {
-    // ------------------------------------------------------------------ epilogue (warps 2..9)
-    const int quarter = warp & 3, half = (warp - 2) >> 2;
+    // ------------------------------------------------------------------ epilogue (warps 3..10)
+    const int quarter = warp & 3, half = (warp - 3) >> 2;
     int acc = 0;
     uint32_t acc_phase = 0;
     bool ok = true;
@@ -638,19 +711,17 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
       int mb, nb_;
       const int tile = item / p.splits;
       tile_coords(tile, p.tiles_m, p.tiles_n, mb, nb_);
-      const float4 bias = p.out_f32 ? load_bias<BN, 32>(p, nb_ * BN, half, lane) : load_bias<BN, epi_group<BN>()>(p, nb_ * BN, half, lane);
-      if (*abort_flag || !mbar_wait(&tfull_bar[acc], acc_phase, p.status, 4)) { ok = false; *abort_flag = 1; break; }
+      const float4 bias = load_bias<BN, (MODE == EPI_F32 || MODE == EPI_F32_ANY) ? 32 : epi_group<BN>()>(p, nb_ * BN, half, lane);
+      if (!wait_or_abort(&tfull_bar[acc], acc_phase, abort_flag, p.status, 4)) { ok = false; *abort_flag = 1; break; }
       tc_fence_after();
       const int row_in_tile = quarter * 32;
       const uint32_t taddr0 = tmem_base + ((uint32_t)row_in_tile << 16) + (uint32_t)(acc * BN);
-      uint8_t* st = epi_stage + (warp - 2) * EPI_STAGE_BYTES;
-      if (p.splits > 1)   // park the fp32 partial tile; splitk_reduce_kernel sums the splits in index order afterwards
-        epilogue_tile_f32<BN>(p, bias, taddr0, st, mb * BM + row_in_tile, nb_ * BN, half, lane,
-                              p.ws + (size_t)item * (BM * BN) + (size_t)row_in_tile * BN);
-      else if (p.out_f32)
-        epilogue_tile_f32<BN>(p, bias, taddr0, st, mb * BM + row_in_tile, nb_ * BN, half, lane, nullptr);
+      uint8_t* st = epi_stage + (warp - 3) * EPI_STAGE_BYTES;
+      if (MODE == EPI_F32 || MODE == EPI_F32_ANY)   // split: park the partial tile; a second kernel sums the splits in order
+        epilogue_groups_f32<BN, MODE>(p, bias, taddr0, st, mb * BM + row_in_tile, nb_ * BN, half, lane,
+                                      p.splits > 1 ? p.ws + (size_t)item * (BM * BN) + (size_t)row_in_tile * BN : nullptr);
       else
-        epilogue_tile_bf16<BN>(p, bias, taddr0, st, mb * BM + row_in_tile, nb_ * BN, half, lane);
+        epilogue_groups_bf16<BN, MODE>(p, bias, taddr0, st, mb * BM + row_in_tile, nb_ * BN, half, lane);
       tc_fence_before();
       __syncwarp();
       if (lane == 0) mbar_arrive(&tempty_bar[acc]);
@@ -722,7 +793,8 @@ __device__ __forceinline__ void umma_commit_pair(uint64_t* bar) {
                : "memory");
 }
 
-__global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(NUM_THREADS, 1)
+template <int MODE>
+__global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(NUM_THREADS2, 1)
 gemm2_bf16_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmB, const GemmParams p) {
   constexpr uint32_t A_BYTES = BM * BK * 2;            // this CTA's 128 rows of A
   constexpr uint32_t B_BYTES = (BN2 / 2) * BK * 2;     // this CTA's 128 of the 256 B columns
@@ -743,7 +815,7 @@ gemm2_bf16_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant
   const int lane = threadIdx.x & 31;
   const uint32_t rank = cluster_ctarank();           // 0 = leader
   const int cluster_id = blockIdx.x >> 1, num_clusters = gridDim.x >> 1;
-  const int num_tiles = p.tiles_m * p.tiles_n;       // tiles of 256 x 256
+  const int num_items = p.tiles_m * p.tiles_n * p.splits;   // tiles of 256 x 256, each in `splits` ranges of k-blocks
 
   if (threadIdx.x == 0) {
     for (int s = 0; s < STAGES2; ++s) {
@@ -776,13 +848,15 @@ gemm2_bf16_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant
       int stage = 0;
       uint32_t phase = 0;
       bool ok = true;
-      for (int tile = cluster_id; tile < num_tiles && ok; tile += num_clusters) {
+      for (int item = cluster_id; item < num_items && ok; item += num_clusters) {
         int mb, nb_;
+        const int tile = item / p.splits, split = item - tile * p.splits;
         tile_coords(tile, p.tiles_m, p.tiles_n, mb, nb_);
+        const int kb0 = split * p.kb_per_split, kb1 = min(p.num_kb, kb0 + p.kb_per_split);
         const int m0 = mb * (2 * BM) + (int)rank * BM;          // this CTA's rows of A
         const int n0 = nb_ * BN2 + (int)rank * (BN2 / 2);       // this CTA's columns of B
-        for (int kb = 0; kb < p.num_kb; ++kb) {
-          if (*abort_flag || !mbar_wait(&empty_bar[stage], phase ^ 1u, p.status, 21)) { ok = false; *abort_flag = 1; break; }
+        for (int kb = kb0; kb < kb1; ++kb) {
+          if (!wait_or_abort(&empty_bar[stage], phase ^ 1u, abort_flag, p.status, 21)) { ok = false; *abort_flag = 1; break; }
           uint8_t* sa = smem + stage * STAGE_BYTES;
           uint8_t* sb = sa + A_BYTES;
           const uint32_t fb = mapa_rank(smem_u32(&full_bar[stage]), 0);
@@ -807,27 +881,29 @@ gemm2_bf16_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant
     // ------------------------------------------------------------------ MMA issuer (leader only)
     if (rank == 0 && elect_one()) {
       const uint32_t idesc = make_idesc(1u, 2 * BM, BN2, (uint32_t)p.a_mn, (uint32_t)p.b_mn);
+      const uint32_t s0 = smem_u32(smem);
+      const uint64_t ad0 = p.a_mn ? make_smem_desc(s0, 64 * BK * 2, 1024, 2) : make_smem_desc(s0, 16, 1024, 2);
+      const uint64_t bd0 = p.b_mn ? make_smem_desc(s0 + A_BYTES, 64 * BK * 2, 1024, 2) : make_smem_desc(s0 + A_BYTES, 16, 1024, 2);
+      const uint32_t astep = (p.a_mn ? UMMA_K * 128 : UMMA_K * 2) >> 4, bstep = (p.b_mn ? UMMA_K * 128 : UMMA_K * 2) >> 4;
       int stage = 0;
       uint32_t phase = 0;
       int acc = 0;
       uint32_t acc_phase = 0;
       bool ok = true;
-      for (int tile = cluster_id; tile < num_tiles && ok; tile += num_clusters) {
-        if (*abort_flag || !mbar_wait(&tempty_bar[acc], acc_phase ^ 1u, p.status, 22)) { ok = false; *abort_flag = 1; break; }
+      for (int item = cluster_id; item < num_items && ok; item += num_clusters) {
+        if (!wait_or_abort(&tempty_bar[acc], acc_phase ^ 1u, abort_flag, p.status, 22)) { ok = false; *abort_flag = 1; break; }
         tc_fence_after();
         const uint32_t d_tmem = tmem_base + (uint32_t)(acc * BN2);
-        for (int kb = 0; kb < p.num_kb; ++kb) {
-          if (*abort_flag || !mbar_wait(&full_bar[stage], phase, p.status, 23)) { ok = false; *abort_flag = 1; break; }
+        const int split = item % p.splits, kb0 = split * p.kb_per_split, kb1 = min(p.num_kb, kb0 + p.kb_per_split);
+        for (int kb = kb0; kb < kb1; ++kb) {
+          if (!wait_or_abort(&full_bar[stage], phase, abort_flag, p.status, 23)) { ok = false; *abort_flag = 1; break; }
           tc_fence_after();
-          const uint32_t sa = smem_u32(smem + stage * STAGE_BYTES);
-          const uint32_t sb = sa + A_BYTES;
+          uint64_t ad = ad0 + (uint32_t)stage * (STAGE_BYTES >> 4), bd = bd0 + (uint32_t)stage * (STAGE_BYTES >> 4);
 #pragma unroll
           for (int k = 0; k < BK / UMMA_K; ++k) {
-            const uint64_t adesc = p.a_mn ? make_smem_desc(sa + k * (UMMA_K * 128), 64 * BK * 2, 1024, 2)
-                                          : make_smem_desc(sa + k * (UMMA_K * 2), 16, 1024, 2);
-            const uint64_t bdesc = p.b_mn ? make_smem_desc(sb + k * (UMMA_K * 128), 64 * BK * 2, 1024, 2)
-                                          : make_smem_desc(sb + k * (UMMA_K * 2), 16, 1024, 2);
-            umma_f16_pair(d_tmem, adesc, bdesc, idesc, (kb | k) != 0 ? 1u : 0u);
+            umma_f16_pair(d_tmem, ad, bd, idesc, ((kb - kb0) | k) != 0 ? 1u : 0u);
+            ad += astep;
+            bd += bstep;
           }
           umma_commit_pair(&empty_bar[stage]);
           if (++stage == STAGES2) { stage = 0; phase ^= 1u; }
@@ -843,17 +919,19 @@ gemm2_bf16_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant
     int acc = 0;
     uint32_t acc_phase = 0;
     bool ok = true;
-    for (int tile = cluster_id; tile < num_tiles && ok; tile += num_clusters) {
+    for (int item = cluster_id; item < num_items && ok; item += num_clusters) {
       int mb, nb_;
-      tile_coords(tile, p.tiles_m, p.tiles_n, mb, nb_);
-      const float4 bias = p.out_f32 ? load_bias<BN2, 32>(p, nb_ * BN2, half, lane) : load_bias<BN2, epi_group<BN2>()>(p, nb_ * BN2, half, lane);
-      if (*abort_flag || !mbar_wait(&tfull_bar[acc], acc_phase, p.status, 24)) { ok = false; *abort_flag = 1; break; }
+      tile_coords(item / p.splits, p.tiles_m, p.tiles_n, mb, nb_);
+      const float4 bias = load_bias<BN2, (MODE == EPI_F32 || MODE == EPI_F32_ANY) ? 32 : epi_group<BN2>()>(p, nb_ * BN2, half, lane);
+      if (!wait_or_abort(&tfull_bar[acc], acc_phase, abort_flag, p.status, 24)) { ok = false; *abort_flag = 1; break; }
       tc_fence_after();
       const int row0 = mb * (2 * BM) + (int)rank * BM + quarter * 32;
       const uint32_t taddr0 = tmem_base + ((uint32_t)(quarter * 32) << 16) + (uint32_t)(acc * BN2);
       uint8_t* st = epi_stage + (warp - 2) * EPI_STAGE_BYTES;
-      if (p.out_f32) epilogue_tile_f32<BN2>(p, bias, taddr0, st, row0, nb_ * BN2, half, lane, nullptr);
-      else epilogue_tile_bf16<BN2>(p, bias, taddr0, st, row0, nb_ * BN2, half, lane);
+      if (MODE == EPI_F32 || MODE == EPI_F32_ANY) epilogue_groups_f32<BN2, MODE>(
+          p, bias, taddr0, st, row0, nb_ * BN2, half, lane,
+          p.splits > 1 ? p.ws + (size_t)item * (2 * BM * BN2) + (size_t)((int)rank * BM + quarter * 32) * BN2 : nullptr);
+      else epilogue_groups_bf16<BN2, MODE>(p, bias, taddr0, st, row0, nb_ * BN2, half, lane);
       tc_fence_before();
       __syncwarp();
       if (lane == 0) mbar_arrive_cluster(mapa_rank(smem_u32(&tempty_bar[acc]), 0));
@@ -879,18 +957,18 @@ __global__ void __launch_bounds__(128)
 splitk_reduce_kernel(const GemmParams p, int BN) {
   const int chunks = BN / 16;
   const long long idx = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-  const long long total = (long long)p.tiles_m * p.tiles_n * BM * chunks;
+  const long long total = (long long)p.tiles_m * p.tiles_n * p.tile_rows * chunks;
   if (idx >= total) return;
   const int c = (int)(idx % chunks);
-  const int row_in_tile = (int)((idx / chunks) % BM);
-  const int tile = (int)(idx / ((long long)chunks * BM));
+  const int row_in_tile = (int)((idx / chunks) % p.tile_rows);
+  const int tile = (int)(idx / ((long long)chunks * p.tile_rows));
   int mb, nb_;
   tile_coords(tile, p.tiles_m, p.tiles_n, mb, nb_);
-  const int row = mb * BM + row_in_tile, col0 = nb_ * BN + c * 16;
+  const int row = mb * p.tile_rows + row_in_tile, col0 = nb_ * BN + c * 16;
   if (row >= p.M || col0 >= p.N) return;
   EpiPrefetch pf;
   epilogue_prefetch16(p, row, col0, true, pf);
-  const size_t tile_elems = (size_t)BM * BN;
+  const size_t tile_elems = (size_t)p.tile_rows * BN;
   const float* src = p.ws + (size_t)tile * p.splits * tile_elems + (size_t)row_in_tile * BN + c * 16;
   float v[16];
 #pragma unroll
@@ -926,16 +1004,16 @@ __global__ void __launch_bounds__(256)
 splitk_reduce_f32_kernel(const GemmParams p, int BN) {
   const int quads = BN / 4;
   const long long idx = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-  const long long total = (long long)p.tiles_m * p.tiles_n * BM * quads;
+  const long long total = (long long)p.tiles_m * p.tiles_n * p.tile_rows * quads;
   if (idx >= total) return;
   const int c = (int)(idx % quads);
-  const int row_in_tile = (int)((idx / quads) % BM);
-  const int tile = (int)(idx / ((long long)quads * BM));
+  const int row_in_tile = (int)((idx / quads) % p.tile_rows);
+  const int tile = (int)(idx / ((long long)quads * p.tile_rows));
   int mb, nb_;
   tile_coords(tile, p.tiles_m, p.tiles_n, mb, nb_);
-  const int row = mb * BM + row_in_tile, col0 = nb_ * BN + c * 4;
+  const int row = mb * p.tile_rows + row_in_tile, col0 = nb_ * BN + c * 4;
   if (row >= p.M || col0 >= p.N) return;
-  const size_t tile_elems = (size_t)BM * BN;
+  const size_t tile_elems = (size_t)p.tile_rows * BN;
   const float* src = p.ws + (size_t)tile * p.splits * tile_elems + (size_t)row_in_tile * BN + c * 4;
   float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
   int sp = 0;
@@ -1018,69 +1096,112 @@ int sm_count() {
   return n;
 }
 
+int g_two_cta_mode = 0;  // 0 = by expected time, 1 = never, 2 = whenever the shape allows it
+
+// ---- choice of tile form and split
+// Time in nanoseconds that a form is expected to take, from measurements on one B200 (graph of ten launches, operands in L2):
+//   * a k-block (64 bf16 of K) costs the issuing threads or the tensor core kb_ns, or the L2 its bytes at about 17 KB/ns over
+//     all SMs, whichever is longer;
+//   * launch, first loads and the last epilogue cost fixed_ns; in further rounds of tiles the epilogue hides behind the next
+//     main loop unless that is shorter (epi_ns);
+//   * a split-K adds a launch and its partial tiles twice through the L2.
+// 4816 x 512 x 3200 (us): 128-column tiles, the earlier choice, 28.6; 256 columns 21.0; pairs 21.5.  512 x 3200 x 4816: 64
+// columns 41.7, 256 in two splits 24.7.  200 x 512 x 512: two splits 7.8, none 5.9.  4096 x 384 x 49152: 64 columns 296,
+// pairs 222, pairs in two splits 145.
+struct TileForm { int bn, rows, kb_bytes, slots, kb_ns, fixed_ns, epi_ns; };   // slots: tiles in flight on 148 SMs
+constexpr TileForm TILE_64 = {64, BM, 24576, 1, 200, 3900, 600}, TILE_128 = {128, BM, 32768, 1, 210, 4600, 900},
+                   TILE_256 = {256, BM, 49152, 1, 280, 4900, 1700}, TILE_PAIR = {256, 2 * BM, 65536, 2, 280, 5300, 1700};
+
+long long form_ns(const TileForm& f, long long tiles, int num_kb, int splits, int sms) {
+  const long long items = tiles * splits, slots = sms / f.slots, waves = ceil_div_ll(items, slots);
+  const long long active = items < slots ? items : slots, l2_ns = active * f.kb_bytes / 17000;
+  const long long loop = (long long)ceil_div(num_kb, splits) * (f.kb_ns > l2_ns ? f.kb_ns : l2_ns);
+  long long t = f.fixed_ns + loop + (waves - 1) * (loop > f.epi_ns ? loop : f.epi_ns);
+  if (splits > 1) t += 2500 + items * f.rows * f.bn * 8 / 5000;
+  return t;
+}
+// Best number of splits of one form; 1 unless the workspace holds the partial tiles.
+long long best_split(const TileForm& f, int M, int N, int num_kb, long long ws_bytes, int sms, int* splits) {
+  const long long tiles = (long long)ceil_div(M, f.rows) * ceil_div(N, f.bn), slots = sms / f.slots;
+  long long best = form_ns(f, tiles, num_kb, 1, sms);
+  *splits = 1;
+  if (tiles * 2 > slots || tiles > NB_GEMM_WS_COUNTERS || num_kb < 8) return best;
+  for (int sp = 2; sp <= num_kb / 4 && tiles * sp <= slots; ++sp) {
+    if (tiles * sp * f.rows * f.bn * 4 > ws_bytes) break;
+    const long long t = form_ns(f, tiles, num_kb, sp, sms);
+    if (t < best) { best = t; *splits = sp; }
+  }
+  return best;
+}
+
+int finish_split(const GemmParams& p, int BN, cudaStream_t stream) {
+  if (p.splits <= 1) return NB_OK;
+  const long long rows = (long long)p.tiles_m * p.tiles_n * p.tile_rows;
+  if (p.out_f32 && !p.bias && !p.act && !p.dact)
+    splitk_reduce_f32_kernel<<<(unsigned)((rows * (BN / 4) + 255) / 256), 256, 0, stream>>>(p, BN);
+  else
+    splitk_reduce_kernel<<<(unsigned)((rows * (BN / 16) + 127) / 128), 128, 0, stream>>>(p, BN);
+  NB_LAUNCH_CHECK();
+  return NB_OK;
+}
+
+// `splits`: wanted number of ranges of k-blocks (the workspace holds their partial tiles)
 template <int BN, int STAGES>
-int launch(const CUtensorMap& tmA, const CUtensorMap& tmB, GemmParams& p, long long ws_bytes, int ws_tiles_cap,
-           cudaStream_t stream) {
+int launch(const CUtensorMap& tmA, const CUtensorMap& tmB, GemmParams& p, int splits, cudaStream_t stream) {
   constexpr size_t smem = (size_t)STAGES * (BM * BK * 2 + BN * BK * 2) + EPI_WARPS * EPI_STAGE_BYTES + 1024 /*align*/ + 256 /*barriers*/;
   static_assert(smem <= 232448, "shared memory budget of one CTA");
-  static bool configured = false;
-  if (!configured) {
-    NB_CUDA(cudaFuncSetAttribute(gemm_bf16_kernel<BN, STAGES>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-    configured = true;
-  }
   p.tiles_m = ceil_div(p.M, BM);
   p.tiles_n = ceil_div(p.N, BN);
+  p.tile_rows = BM;
   p.num_kb = ceil_div(p.K, p.tf32 ? BK / 2 : BK);
-  const int tiles = p.tiles_m * p.tiles_n;
-  // split-K when the tile count leaves most SMs idle and K is deep: each split keeps >= 4 k-blocks
-  int splits = 1;
-  if (p.ws && p.tile_ctr && tiles * 2 <= sm_count() && p.num_kb >= 8 && tiles <= ws_tiles_cap) {
-    splits = sm_count() / tiles;
-    if (splits > p.num_kb / 4) splits = p.num_kb / 4;
-    const long long cap = ws_bytes / ((long long)tiles * BM * BN * 4);
-    if (splits > cap) splits = (int)cap;
-    if (splits < 1) splits = 1;
-  }
   p.kb_per_split = ceil_div(p.num_kb, splits);
   p.splits = ceil_div(p.num_kb, p.kb_per_split);
-  const int items = tiles * p.splits;
+  const int items = p.tiles_m * p.tiles_n * p.splits;
   const int grid = items < sm_count() ? items : sm_count();
-  gemm_bf16_kernel<BN, STAGES><<<grid, NUM_THREADS, smem, stream>>>(tmA, tmB, p);
-  NB_LAUNCH_CHECK();
-  if (p.splits > 1) {
-    if (p.out_f32 && !p.bias && !p.act && !p.dact) {
-      const long long threads = (long long)tiles * BM * (BN / 4);
-      splitk_reduce_f32_kernel<<<(unsigned)((threads + 255) / 256), 256, 0, stream>>>(p, BN);
-    } else {
-      const long long threads = (long long)tiles * BM * (BN / 16);
-      splitk_reduce_kernel<<<(unsigned)((threads + 127) / 128), 128, 0, stream>>>(p, BN);
-    }
-    NB_LAUNCH_CHECK();
+  typedef void (*Kernel)(CUtensorMap, CUtensorMap, GemmParams);
+  // narrow tiles (heads of a few columns) run the general epilogues only
+  static const Kernel kernels[EPI_MODES] = {
+      gemm_bf16_kernel<BN, STAGES, BN < 64 ? EPI_BF16 : EPI_PLAIN>, gemm_bf16_kernel<BN, STAGES, BN < 64 ? EPI_BF16 : EPI_RELU>,
+      gemm_bf16_kernel<BN, STAGES, BN < 64 ? EPI_BF16 : EPI_GELU>,  gemm_bf16_kernel<BN, STAGES, BN < 64 ? EPI_BF16 : EPI_ADD>,
+      gemm_bf16_kernel<BN, STAGES, EPI_BF16>,                       gemm_bf16_kernel<BN, STAGES, EPI_F32>,
+      gemm_bf16_kernel<BN, STAGES, EPI_F32_ANY>};
+  static bool configured[EPI_MODES] = {};
+  const EpiMode mode = epi_mode(p, p.splits > 1);
+  if (!configured[mode]) {
+    NB_CUDA(cudaFuncSetAttribute(kernels[mode], cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    configured[mode] = true;
   }
-  return NB_OK;
+  kernels[mode]<<<grid, NUM_THREADS, smem, stream>>>(tmA, tmB, p);
+  NB_LAUNCH_CHECK();
+  return finish_split(p, BN, stream);
 }
 
-int launch_two_cta(const CUtensorMap& tmA, const CUtensorMap& tmB, GemmParams& p, cudaStream_t stream) {
+int launch_two_cta(const CUtensorMap& tmA, const CUtensorMap& tmB, GemmParams& p, int splits, cudaStream_t stream) {
   constexpr size_t smem = (size_t)STAGES2 * (BM * BK * 2 + (BN2 / 2) * BK * 2) + EPI_WARPS * EPI_STAGE_BYTES + 1024 /*align*/ + 256 /*barriers*/;
   static_assert(smem <= 232448, "shared memory budget of one CTA");
-  static bool configured = false;
-  if (!configured) {
-    NB_CUDA(cudaFuncSetAttribute(gemm2_bf16_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-    configured = true;
-  }
   p.tiles_m = ceil_div(p.M, 2 * BM);
   p.tiles_n = ceil_div(p.N, BN2);
+  p.tile_rows = 2 * BM;
   p.num_kb = ceil_div(p.K, BK);
-  p.splits = 1;
-  p.kb_per_split = p.num_kb;
-  const int tiles = p.tiles_m * p.tiles_n;
-  const int clusters = tiles < sm_count() / 2 ? tiles : sm_count() / 2;
-  gemm2_bf16_kernel<<<2 * clusters, NUM_THREADS, smem, stream>>>(tmA, tmB, p);
+  p.kb_per_split = ceil_div(p.num_kb, splits);
+  p.splits = ceil_div(p.num_kb, p.kb_per_split);
+  const int items = p.tiles_m * p.tiles_n * p.splits;
+  const int clusters = items < sm_count() / 2 ? items : sm_count() / 2;
+  typedef void (*Kernel)(CUtensorMap, CUtensorMap, GemmParams);
+  static const Kernel kernels[EPI_MODES] = {gemm2_bf16_kernel<EPI_PLAIN>, gemm2_bf16_kernel<EPI_RELU>, gemm2_bf16_kernel<EPI_GELU>,
+                                            gemm2_bf16_kernel<EPI_ADD>,   gemm2_bf16_kernel<EPI_BF16>, gemm2_bf16_kernel<EPI_F32>,
+                                            gemm2_bf16_kernel<EPI_F32_ANY>};
+  static bool configured[EPI_MODES] = {};
+  const EpiMode mode = epi_mode(p, p.splits > 1);
+  if (!configured[mode]) {
+    NB_CUDA(cudaFuncSetAttribute(kernels[mode], cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    configured[mode] = true;
+  }
+  kernels[mode]<<<2 * clusters, NUM_THREADS2, smem, stream>>>(tmA, tmB, p);
   NB_LAUNCH_CHECK();
-  return NB_OK;
+  return finish_split(p, BN2, stream);
 }
 
-int g_two_cta_mode = 0;  // 0 = by problem size, 1 = never, 2 = whenever the shape allows it
 
 }  // namespace
 
@@ -1104,25 +1225,33 @@ static int gemm_any(int tf32, const void* A, const void* B, void* D, int M, int 
   const int elt = tf32 ? 4 : 2, bk = 128 / elt;   // elements per 128-byte row = k-block depth = MN-major chunk width
   if (accumulate && !out_f32) return NB_ERR_BAD_ARG;
   if (dact && !aux) return NB_ERR_BAD_ARG;
-  int BN = bn_hint;
-  if (BN == 0) {
-    // widest tile that still gives every SM work; MN-major B needs whole 64-column boxes
-    BN = 128;
-    const long long t128 = (long long)ceil_div(M, BM) * ceil_div(N, 128);
-    if (N <= 64 || t128 < sm_count()) BN = 64;
-    if (N >= 256 && (long long)ceil_div(M, BM) * ceil_div(N, 256) >= 2LL * sm_count()) BN = 256;
-    if (!b_mn) {
-      if (N <= 16) BN = 16;
-      else if (N <= 32) BN = 32;
-    }
-  }
-  if (b_mn && BN < bk) BN = bk;
-  // two-CTA tiles once the 256 x 256 tiles keep about two thirds of the SM pairs busy (measured: 2048 x 2048 x 16384,
-  // 64 tiles on 74 pairs, runs 1.74x faster this way than as split-K one-CTA tiles)
+  // workspace layout: [NB_GEMM_WS_COUNTERS u32 tile counters (zero at rest)] [fp32 partial tiles]
+  const bool have_ws = workspace && workspace_bytes > NB_GEMM_WS_COUNTERS * 4 + (1 << 20);
+  const long long ws_bytes = have_ws ? workspace_bytes - NB_GEMM_WS_COUNTERS * 4 : 0;
+  const int num_kb = ceil_div(K, bk), sms = sm_count();
+  int BN = bn_hint, splits = 1;
   bool two_cta = false;
-  if (!tf32 && bn_hint == 0 && g_two_cta_mode != 1 && M >= 256 && N >= 256 && K >= 128) {
-    const long long t2 = (long long)ceil_div(M, 2 * BM) * ceil_div(N, BN2);
-    two_cta = g_two_cta_mode == 2 || t2 * 3 >= (long long)sm_count();
+  if (b_mn && BN && BN < bk) BN = bk;
+  if (BN == 0 && N <= 32 && !b_mn) {
+    BN = N <= 16 ? 16 : 32;                        // heads of a few columns
+    best_split(TILE_64, M, N, num_kb, ws_bytes, sms, &splits);
+  } else if (BN == 0) {
+    // the form with the smallest expected time; MN-major B needs whole 64-column boxes
+    long long best = best_split(TILE_64, M, N, num_kb, ws_bytes, sms, &splits);
+    BN = 64;
+    int sp;
+    for (const TileForm* f : {&TILE_128, &TILE_256}) {
+      if (N <= f->bn / 2) break;
+      const long long t = best_split(*f, M, N, num_kb, ws_bytes, sms, &sp);
+      if (t < best) { best = t; BN = f->bn; splits = sp; }
+    }
+    if (!tf32 && g_two_cta_mode != 1 && M >= 256 && N >= 256 && K >= 128) {
+      const long long t = best_split(TILE_PAIR, M, N, num_kb, ws_bytes, sms, &sp);
+      if (t < best || g_two_cta_mode == 2) { two_cta = true; splits = sp; }
+    }
+  } else {
+    const TileForm f = BN == 256 ? TILE_256 : (BN == 128 ? TILE_128 : TILE_64);
+    best_split(TileForm{BN, BM, f.kb_bytes, 1, f.kb_ns, f.fixed_ns, f.epi_ns}, M, N, num_kb, ws_bytes, sms, &splits);
   }
   if (two_cta) BN = BN2 / 2;   // the B box of one CTA
   CUtensorMap tmA, tmB;
@@ -1141,23 +1270,16 @@ static int gemm_any(int tf32, const void* A, const void* B, void* D, int M, int 
   p.alpha = alpha;
   p.D = D; p.bias = bias; p.aux = (const __nv_bfloat16*)aux; p.status = status;
   p.conv = 0;
-  // workspace layout: [NB_GEMM_WS_COUNTERS u32 tile counters (zero at rest)] [fp32 partial tiles]
-  long long ws_bytes = 0;
-  p.ws = nullptr;
-  p.tile_ctr = nullptr;
-  if (workspace && workspace_bytes > NB_GEMM_WS_COUNTERS * 4 + (1 << 20)) {
-    p.tile_ctr = (unsigned int*)workspace;
-    p.ws = (float*)((char*)workspace + NB_GEMM_WS_COUNTERS * 4);
-    ws_bytes = workspace_bytes - NB_GEMM_WS_COUNTERS * 4;
-  }
+  p.ws = have_ws ? (float*)((char*)workspace + NB_GEMM_WS_COUNTERS * 4) : nullptr;
+  p.tile_ctr = have_ws ? (unsigned int*)workspace : nullptr;
   cudaStream_t s = (cudaStream_t)stream;
-  if (two_cta) return launch_two_cta(tmA, tmB, p, s);
+  if (two_cta) return launch_two_cta(tmA, tmB, p, splits, s);
   switch (BN) {
-    case 256: return launch<256, 4>(tmA, tmB, p, ws_bytes, NB_GEMM_WS_COUNTERS, s);
-    case 128: return launch<128, 6>(tmA, tmB, p, ws_bytes, NB_GEMM_WS_COUNTERS, s);
-    case 64: return launch<64, 8>(tmA, tmB, p, ws_bytes, NB_GEMM_WS_COUNTERS, s);
-    case 32: return launch<32, 8>(tmA, tmB, p, ws_bytes, NB_GEMM_WS_COUNTERS, s);
-    case 16: return launch<16, 8>(tmA, tmB, p, ws_bytes, NB_GEMM_WS_COUNTERS, s);
+    case 256: return launch<256, 4>(tmA, tmB, p, splits, s);
+    case 128: return launch<128, 6>(tmA, tmB, p, splits, s);
+    case 64: return launch<64, 8>(tmA, tmB, p, splits, s);
+    case 32: return launch<32, 8>(tmA, tmB, p, splits, s);
+    case 16: return launch<16, 8>(tmA, tmB, p, splits, s);
     default: return NB_ERR_BAD_ARG;
   }
 }
@@ -1220,8 +1342,8 @@ int nb_conv_implicit_fwd(const void* x, const void* Wt, void* y, int B, int H, i
   p.conv = 1; p.conv_c = C; p.conv_ow = OW; p.conv_oh = OH; p.conv_kw = KW; p.conv_pad = pad; p.conv_bw = bw;
   p.conv_taps = KH * KW; p.conv_b = B;
   cudaStream_t s = (cudaStream_t)stream;
-  if (BN == 128) return launch<128, 6>(tmA, tmB, p, 0, 0, s);
-  return launch<64, 8>(tmA, tmB, p, 0, 0, s);
+  if (BN == 128) return launch<128, 6>(tmA, tmB, p, 1, s);
+  return launch<64, 8>(tmA, tmB, p, 1, s);
 }
 
 
@@ -1271,8 +1393,10 @@ int nb_conv_implicit_wgrad(const void* x, const void* dy, float* dW, int B, int 
   p.conv = 2; p.conv_c = C; p.conv_ow = OW; p.conv_oh = OH; p.conv_kw = KW; p.conv_pad = pad; p.conv_bw = bw;
   p.conv_taps = KH * KW; p.conv_b = B;
   cudaStream_t s = (cudaStream_t)stream;
-  if (BN == 128) return launch<128, 6>(tmA, tmB, p, ws_bytes, NB_GEMM_WS_COUNTERS, s);
-  return launch<64, 8>(tmA, tmB, p, ws_bytes, NB_GEMM_WS_COUNTERS, s);
+  int splits;
+  best_split(BN == 128 ? TILE_128 : TILE_64, Kc, OC, ceil_div(Mpix, BK), ws_bytes, sm_count(), &splits);
+  if (BN == 128) return launch<128, 6>(tmA, tmB, p, splits, s);
+  return launch<64, 8>(tmA, tmB, p, splits, s);
 }
 
 }  // extern "C"

@@ -1,5 +1,6 @@
-// Convolution support kernels for the NHWC bf16 path: patch gather (im2col) feeding the tcgen05 GEMM,
-// its adjoint as a deterministic gather (no atomics), BatchNorm2D in training mode (per-channel batch
+// Convolution support kernels for the NHWC bf16 path: patch matrix (im2col) for transposed convolutions and for callers that
+// ask for it (the convolution itself gathers its patches, conv_gemm_tcgen05.cu), its adjoint as a deterministic gather (no
+// atomics) for strided data gradients, BatchNorm2D in training mode (per-channel batch
 // statistics, fused scale/shift/ReLU/residual), max pooling, and the uint8 camera-image normaliser.
 //
 // A convolution is  Y[B·OH·OW, OC] = col[B·OH·OW, KH·KW·C] · W[KH·KW·C, OC]  with the bias / ReLU in the GEMM
@@ -36,34 +37,26 @@ im2col_kernel(const __nv_bfloat16* __restrict__ x, __nv_bfloat16* __restrict__ c
   }
 }
 
-// dx[b, h, w, c] = Σ_{kh,kw : (h+p-kh) % s == 0, ...} dcol[b, oh, ow, kh, kw, c]   (gather: one writer per element)
+// dx[b, h, w, c] = Σ_{kh,kw : (h+p-kh) % s == 0, ...} dcol[b, oh, ow, kh, kw, c]   (gather: one writer per element).  A block owns
+// part of one input row, a thread 8 channels of a pixel; only the taps of the pixel's residue modulo the stride are visited.
+// 19200 x 1152 -> 16 x 60 x 80 x 128 (44 MB read, 20 MB written): 25.5 us with 64-bit divisions and all taps tested, 14.3 now.
 __global__ void __launch_bounds__(256)
-col2im_kernel(const __nv_bfloat16* __restrict__ dcol, __nv_bfloat16* __restrict__ dx, int B, int H, int W, int C, int KH,
-              int KW, int stride, int pad, int OH, int OW, int ldc) {
-  const int cv = C / 8;
-  const long long total = (long long)B * H * W * cv;
-  const long long step = (long long)gridDim.x * blockDim.x;
-  for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < total; i += step) {
-    const int c8 = (int)(i % cv);
-    long long r = i / cv;
-    const int w = (int)(r % W); r /= W;
-    const int h = (int)(r % H);
-    const int b = (int)(r / H);
+col2im_kernel(const __nv_bfloat16* __restrict__ dcol, __nv_bfloat16* __restrict__ dx, int H, int W, int C, int KH, int KW,
+              int stride, int pad, int OH, int OW, int ldc) {
+  const int cv = C / 8, b = blockIdx.x / H, h = blockIdx.x - b * H;
+  for (int i = blockIdx.y * 256 + threadIdx.x; i < W * cv; i += gridDim.y * 256) {
+    const int w = i / cv, c8 = i - w * cv;
     float acc[8];
 #pragma unroll
     for (int k = 0; k < 8; ++k) acc[k] = 0.f;
-    for (int kh = 0; kh < KH; ++kh) {
-      const int th = h + pad - kh;
-      if (th < 0 || th % stride) continue;
-      const int oh = th / stride;
-      if (oh >= OH) continue;
-      for (int kw = 0; kw < KW; ++kw) {
-        const int tw = w + pad - kw;
-        if (tw < 0 || tw % stride) continue;
-        const int ow = tw / stride;
-        if (ow >= OW) continue;
+    const int th = h + pad, tw = w + pad;
+    // the last output row / column whose window starts at or before this pixel, then backwards through the windows
+    for (int oh = min(OH - 1, th / stride); oh >= 0 && th - oh * stride < KH; --oh) {
+      const int kh = th - oh * stride;
+      for (int ow = min(OW - 1, tw / stride); ow >= 0 && tw - ow * stride < KW; --ow) {
+        const int kw = tw - ow * stride;
         const size_t m = ((size_t)b * OH + oh) * OW + ow;
-        const uint4 v = *reinterpret_cast<const uint4*>(dcol + m * ldc + ((size_t)kh * KW + kw) * C + c8 * 8);
+        const uint4 v = __ldg(reinterpret_cast<const uint4*>(dcol + m * ldc + ((size_t)kh * KW + kw) * C + c8 * 8));
         const __nv_bfloat162* hp = reinterpret_cast<const __nv_bfloat162*>(&v);
 #pragma unroll
         for (int k = 0; k < 4; ++k) {
@@ -604,8 +597,8 @@ int nb_im2col(const void* x, void* col, int B, int H, int W, int C, int KH, int 
 int nb_col2im(const void* dcol, void* dx, int B, int H, int W, int C, int KH, int KW, int stride, int pad, int OH, int OW,
               int ldc, void* stream) {
   if (C % 8 || ldc % 8) return NB_ERR_UNALIGNED;
-  col2im_kernel<<<g1((long long)B * H * W * (C / 8)), 256, 0, (cudaStream_t)stream>>>(
-      (const __nv_bfloat16*)dcol, (__nv_bfloat16*)dx, B, H, W, C, KH, KW, stride, pad, OH, OW, ldc);
+  col2im_kernel<<<dim3((unsigned)(B * H), pool_blocks(W * (C / 8))), 256, 0, (cudaStream_t)stream>>>(
+      (const __nv_bfloat16*)dcol, (__nv_bfloat16*)dx, H, W, C, KH, KW, stride, pad, OH, OW, ldc);
   NB_LAUNCH_CHECK();
   return NB_OK;
 }

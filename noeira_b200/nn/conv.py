@@ -31,16 +31,20 @@ def _scratch(device, n):
     return t
 
 
+def _aligned(t):
+    """``t`` contiguous with a 16-byte aligned base (16-byte copies of 8 channels)."""
+    t = t if t.is_contiguous() else t.contiguous()
+    return t if t.data_ptr() % 16 == 0 else t.clone()
+
+
 class Conv2D(Module):
     def __init__(self, ic, oc, k, stride=1, pad=0, bias=True, relu=False, need_input_grad=True):
         super().__init__()
         self.ic, self.oc, self.k, self.stride, self.pad, self.relu = ic, oc, k, stride, pad, relu
         self.icp = (ic + 7) // 8 * 8          # channels as stored (stem: 3 → 8, extra channels are zero)
         self.need_input_grad = need_input_grad
-        self.force_implicit = False
+        # False: patch matrix in memory (im2col) instead of the gathering convolution kernel
         self.implicit_gemm = os.environ.get("NOEIRA_B200_IMPLICIT_CONV", "1") != "0"
-        # weight gradient straight from the NHWC input (no patch matrix in the backward either)
-        self.implicit_wgrad = os.environ.get("NOEIRA_B200_IMPLICIT_WGRAD", "0") == "1"
         self.weight = self.add_param("weight", (k * k * self.icp, oc), decay=True, init=Kaiming(), fan_in=ic * k * k,
                                      fan_out=oc)
         if self.icp != ic:
@@ -53,17 +57,14 @@ class Conv2D(Module):
                                                                   (0, 0, 0, icp - ic)).reshape(KK * KK * icp, oc)
 
     def _implicit_ok(self, C, OW):
-        if self.stride != 1 or C % 64 or not self.implicit_gemm:
+        """The gathering kernel takes every stride, padding and width; its offsets are 32-bit."""
+        if not self.implicit_gemm or C % 8:
             return False
-        # a trainable layer needs the patch matrix for its weight gradient anyway; building it in the forward and
-        # reusing it measured 0.3 ms faster per ACT step than implicit forward + rebuild in the backward
-        if self.training and torch.is_grad_enabled() and not self.weight.frozen and not self.force_implicit \
-                and not (self.implicit_wgrad and self._implicit_wgrad_ok(OW)):
-            return False
-        bw = 1
-        while bw < 128 and OW % (bw * 2) == 0:
-            bw *= 2
-        return bw >= 16          # runs of 8 pixels need 16 TMA boxes per stage and measured slower than the patch matrix
+        B, H, W = getattr(self, "_in", (1, 1, 1))
+        return (B * H + 2 * self.pad) * (W + 2 * self.pad) * C < 1 << 31 and B * (H + 2 * self.pad) * OW < (1 << 31) - 256
+
+    def _implicit_wgrad_ok(self, OW):
+        return self._implicit_ok(self.icp, OW)
 
     def _patches(self):
         """Patch matrix [B·OH·OW, KH·KW·C] of the saved input (backward of the implicit-GEMM forward)."""
@@ -71,7 +72,7 @@ class Conv2D(Module):
         B, H, W, C = x.shape
         OH, OW = self.out_hw(H, W)
         K = self.k * self.k * C
-        if self.k == 1 and self.pad == 0:
+        if self._pointwise:
             return x.reshape(B * OH * OW, C)
         col = torch.empty(B * OH * OW, K, device=x.device, dtype=torch.bfloat16)
         check(cuda_lib().nb_im2col(ptr(x), ptr(col), *(ctypes.c_int(v) for v in (B, H, W, C, self.k, self.k, self.stride,
@@ -94,28 +95,26 @@ class Conv2D(Module):
             self._y = torch.relu(y) if self.relu else y
             return self._y
         M, K = B * OH * OW, self.k * self.k * C
-        if self._implicit_ok(C, OW):
-            # implicit GEMM: the GEMM's TMA producer reads the patches straight from x (no patch matrix in memory);
-            # the backward pass rebuilds the patch matrix only if a weight gradient is needed
-            xc = x if x.is_contiguous() else x.contiguous()
-            y = torch.empty(M, self.weight.shadow.shape[1], device=x.device, dtype=torch.bfloat16)
-            from ..ops.status import device_status
-            from ..ops.gemm import ACT
-            check(cuda_lib().nb_conv_implicit_fwd(ptr(xc), ptr(self.weight.shadow), ptr(y), *(ctypes.c_int(v) for v in (
-                B, H, W, C, self.oc, self.k, self.k, self.pad, self.weight.shadow.stride(0), y.stride(0))),
-                ptr(self.bias.storage if self.bias is not None else None), ctypes.c_int(ACT["relu" if self.relu else None]),
-                None, ctypes.c_int(0), ptr(device_status(x.device)), stream_ptr()), "conv_implicit_fwd")
-            self._col, self._xin, self._y = None, xc, y
-            return y[:, : self.oc].reshape(B, OH, OW, self.oc) if y.shape[1] != self.oc else y.view(B, OH, OW, self.oc)
-        self._xin = None
-        if self.k == 1 and self.stride == 1 and self.pad == 0:
+        self._col, self._xin = None, None
+        if self._pointwise:
             col = x.reshape(M, C)
+            if self.implicit_gemm:
+                self._xin = x                      # the input is its own patch matrix
+        elif self._implicit_ok(C, OW):
+            # the convolution kernel gathers the patches straight from x: no patch matrix in either direction
+            xc = _aligned(x)
+            y = torch.empty(M, self.weight.shadow.shape[1], device=x.device, dtype=torch.bfloat16)
+            self._conv(xc, self.weight.shadow, y, self.oc, self.stride, self.pad, False,
+                       self.bias.storage if self.bias is not None else None, "relu" if self.relu else None)
+            self._xin, self._y = xc, y
+            return y[:, : self.oc].reshape(B, OH, OW, self.oc) if y.shape[1] != self.oc else y.view(B, OH, OW, self.oc)
         else:
             col = torch.empty(M, K, device=x.device, dtype=torch.bfloat16)
             xc = x if x.is_contiguous() else x.contiguous()
             check(cuda_lib().nb_im2col(ptr(xc), ptr(col), *(ctypes.c_int(v) for v in (B, H, W, C, self.k, self.k, self.stride,
                                                                                    self.pad, OH, OW, K)), stream_ptr()), "im2col")
-        self._col = col
+        if self._xin is None:
+            self._col = col
         y = ops.gemm(col, self.weight.shadow, b_mn=True, bias=self.bias.storage if self.bias is not None else None,
                      act="relu" if self.relu else None)
         self._y = y
@@ -145,7 +144,7 @@ class Conv2D(Module):
             from .layers import act_backward
             d2 = act_backward(d2.contiguous(), self._y[:, : self.oc].contiguous() if self._y.shape[1] != self.oc else self._y, "relu")
         if not self.weight.frozen:
-            if self._col is None and self._xin is not None and self.implicit_wgrad and self._implicit_wgrad_ok(OW):
+            if self._col is None and not self._pointwise and self._implicit_wgrad_ok(OW):
                 self._implicit_wgrad(d2, B, H, W)
             else:
                 col = self._col if self._col is not None else self._patches()
@@ -158,52 +157,51 @@ class Conv2D(Module):
             return self._implicit_dgrad(d2, B, H, W, OH, OW)
         K = self.k * self.k * self.icp
         dcol = ops.gemm(d2, self.weight.shadow[:, : self.oc])           # [M, K]
-        if self.k == 1 and self.stride == 1 and self.pad == 0:
+        if self._pointwise:
             return dcol.view(B, H, W, self.icp)
         dx = torch.empty(B, H, W, self.icp, device=dy.device, dtype=torch.bfloat16)
         check(cuda_lib().nb_col2im(ptr(dcol), ptr(dx), *(ctypes.c_int(v) for v in (B, H, W, self.icp, self.k, self.k, self.stride,
                                                                                self.pad, OH, OW, K)), stream_ptr()), "col2im")
         return dx
 
-    def _implicit_wgrad_ok(self, OW):
-        bw = 1
-        while bw < 64 and OW % (bw * 2) == 0:
-            bw *= 2
-        return self.stride == 1 and self.icp % 64 == 0 and bw >= 8
+    @property
+    def _pointwise(self):
+        return self.k == 1 and self.stride == 1 and self.pad == 0
+
+    def _conv(self, x, w, y, oc, stride, pad, mirror, bias=None, act=None):
+        from ..ops.gemm import ACT, default_workspace
+        from ..ops.status import device_status
+        B, H, W, C = x.shape
+        ws = default_workspace(x.device)
+        check(cuda_lib().nb_conv_gemm(ptr(x), ptr(w), ptr(y), *(ctypes.c_int(v) for v in (
+            B, H, W, C, oc, self.k, self.k, stride, pad, int(mirror), w.stride(0), y.stride(0))), ptr(bias), ctypes.c_int(ACT[act]),
+            ptr(device_status(x.device)), ptr(ws), ctypes.c_longlong(ws.numel()), stream_ptr()), "conv_gemm")
 
     def _implicit_wgrad(self, d2, B, H, W):
-        """dW += patches(x)ᵀ · dy with the patches read by the GEMM's TMA producer from the saved NHWC input."""
+        """dW += patches(x)ᵀ · dy with the patches gathered from the saved NHWC input."""
         from ..ops.gemm import default_workspace
         from ..ops.status import device_status
         x, g = self._xin, self.weight.grad_storage
-        d2 = d2 if (d2.stride(0) * 2) % 16 == 0 and d2.data_ptr() % 16 == 0 else d2.contiguous()
+        if (d2.stride(0) * 2) % 16 or d2.data_ptr() % 16:
+            d2 = d2.contiguous()
         ws = default_workspace(x.device)
-        check(cuda_lib().nb_conv_implicit_wgrad(ptr(x), ptr(d2), ptr(g), *(ctypes.c_int(v) for v in (
-            B, H, W, self.icp, self.oc, self.k, self.k, self.pad, d2.stride(0), g.stride(0))), ptr(device_status(x.device)),
-            ptr(ws), ctypes.c_longlong(ws.numel()), stream_ptr()), "conv_implicit_wgrad")
+        check(cuda_lib().nb_conv_gemm_wgrad(ptr(x), ptr(d2), ptr(g), *(ctypes.c_int(v) for v in (
+            B, H, W, self.icp, self.oc, self.k, self.k, self.stride, self.pad, d2.stride(0), g.stride(0))), ptr(device_status(x.device)),
+            ptr(ws), ctypes.c_longlong(ws.numel()), stream_ptr()), "conv_gemm_wgrad")
 
     def _implicit_dgrad_ok(self, W):
-        """Stride-1 layers with at least 64 output channels: the input gradient is itself a stride-1 convolution of
-        dy (taps mirrored, channel roles swapped), which the implicit-GEMM kernel computes without the 9x larger
-        patch-gradient matrix and the col2im pass over it."""
-        if self.stride != 1 or self.k == 1 or self.oc % 64 or not self.implicit_gemm or 2 * self.pad > self.k - 1 + self.k - 1:
+        """Stride-1 layers whose output channels fill 64-wide k-blocks: the input gradient is itself a stride-1 convolution of
+        dy (taps mirrored, channel roles swapped), without the k² times larger patch-gradient matrix and the pass over it."""
+        if self.stride != 1 or self.k == 1 or self.oc % 64 or not self.implicit_gemm or self.pad > self.k - 1:
             return False
-        bw = 1
-        while bw < 128 and W % (bw * 2) == 0:
-            bw *= 2
-        return bw >= 8
+        B, H, _ = getattr(self, "_in", (1, 1, 1))
+        return (B * H + 4 * self.k) * (W + 4 * self.k) * max(self.oc, self.icp) < 1 << 31
 
     def _implicit_dgrad(self, d2, B, H, W, OH, OW):
-        k, oc, icp = self.k, self.oc, self.icp
-        # W'[(kh', kw', oc), ic] = W[(k-1-kh', k-1-kw', ic), oc]
-        wt = self.weight.shadow[:, :oc].reshape(k, k, icp, oc).flip(0, 1).permute(0, 1, 3, 2).contiguous().view(k * k * oc, icp)
-        dyc = d2 if d2.is_contiguous() else d2.contiguous()
-        dx = torch.empty(B * H * W, icp, device=d2.device, dtype=torch.bfloat16)
-        from ..ops.status import device_status
-        check(cuda_lib().nb_conv_implicit_fwd(ptr(dyc), ptr(wt), ptr(dx), *(ctypes.c_int(v) for v in (
-            B, OH, OW, oc, icp, k, k, k - 1 - self.pad, wt.stride(0), dx.stride(0))), None, ctypes.c_int(0), None,
-            ctypes.c_int(0), ptr(device_status(d2.device)), stream_ptr()), "conv_implicit_dgrad")
-        return dx.view(B, H, W, icp)
+        dyc = _aligned(d2).view(B, OH, OW, self.oc)
+        dx = torch.empty(B * H * W, self.icp, device=d2.device, dtype=torch.bfloat16)
+        self._conv(dyc, self.weight.shadow, dx, self.icp, 1, self.k - 1 - self.pad, True)
+        return dx.view(B, H, W, self.icp)
 
     def _release(self):
         self._col = self._y = self._xin = None

@@ -156,9 +156,29 @@ def cuda_lib() -> ctypes.CDLL:
             build()
         if not lib.exists():
             raise RuntimeError(f"{lib} is missing: run `python -m noeira_b200.build`")
-        _cuda = ctypes.CDLL(str(lib))
-        _cuda._bounds_registered = set()
+        loaded = ctypes.CDLL(str(lib))
+        loaded._bounds_registered = set()
+        for name, sig in _SIGNATURES.items():
+            getattr(loaded, name).argtypes = [_CTYPES[c] for c in sig]
+        _cuda = loaded
     return _cuda
+
+
+# Argument types of the launchers that inference and training call most: with them declared a call site passes plain ints
+# (pointers as ``tensor.data_ptr()``, None for NULL) and ctypes converts them in C.  Wrapping each of a GEMM's 25 arguments in
+# a ctypes object, and asking torch for a Stream object per launch, took most of the 31 us that a launch cost the host; the
+# 345 launches of one ACT policy query were bound by it (5.8 ms of host time per query, 4.0 with both changes).
+_CTYPES = {"p": ctypes.c_void_p, "i": ctypes.c_int, "l": ctypes.c_longlong, "f": ctypes.c_float}
+_GEMM_SIG = "ppp" + "i" * 10 + "fpipiipiplp"
+_SIGNATURES = {
+    "nb_gemm_bf16": _GEMM_SIG, "nb_gemm_tf32": _GEMM_SIG,
+    "nb_conv_gemm": "ppp" + "i" * 12 + "pipplp",
+    "nb_conv_gemm_wgrad": "ppp" + "i" * 11 + "pplp",
+    "nb_flash_attn_fwd": "ppppp" + "i" * 6 + "l" * 10 + "fiiipppp",
+    "nb_norm_fwd": "pipppip" + "iifip",
+    "nb_bn_fwd": "pppppppppp" + "liffiip",
+    "nb_act_fwd": "pplip", "nb_act_bwd": "ppplip",
+}
 
 
 def register_bounds_status(status_tensor) -> int:
@@ -222,7 +242,18 @@ def ptr(t) -> ctypes.c_void_p:
     return ctypes.c_void_p(t.data_ptr())
 
 
+_RAW_STREAM = None
+
+
+def raw_stream() -> int:
+    """Handle of the current stream of the current device, without the Stream object torch would build around it."""
+    global _RAW_STREAM
+    if _RAW_STREAM is None:
+        import torch
+        torch.cuda.current_stream()                       # initialises CUDA
+        _RAW_STREAM = (torch._C._cuda_getCurrentRawStream, torch._C._cuda_getDevice)
+    return _RAW_STREAM[0](_RAW_STREAM[1]())
+
+
 def stream_ptr(stream=None) -> ctypes.c_void_p:
-    import torch
-    s = stream if stream is not None else torch.cuda.current_stream()
-    return ctypes.c_void_p(s.cuda_stream)
+    return ctypes.c_void_p(stream.cuda_stream if stream is not None else raw_stream())

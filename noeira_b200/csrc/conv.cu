@@ -226,16 +226,22 @@ bn_bwd_finish_kernel(const float* __restrict__ p0, const float* __restrict__ p1,
   if (dbeta) dbeta[c] += s;
 }
 
-// y = relu?( (x - mean) * rstd * gamma + beta + residual? )
+// y = relu?( (x - mean) * rstd * gamma + beta + residual? ); rstd null: from `var` (inference with running statistics)
 __global__ void __launch_bounds__(256)
 bn_apply_kernel(const __nv_bfloat16* __restrict__ x, const float* __restrict__ mean, const float* __restrict__ rstd,
-                const float* __restrict__ gamma, const float* __restrict__ beta, const __nv_bfloat16* __restrict__ res,
+                const float* __restrict__ var, float eps, const float* __restrict__ gamma, const float* __restrict__ beta, const __nv_bfloat16* __restrict__ res,
                 __nv_bfloat16* __restrict__ y, long long M, int C, int relu) {
   const BnMap m = bn_map(C, blockIdx.x, gridDim.x);
   if (!m.active) return;
   float mu[8], rs[8], ga[8], be[8];
   load8f(mean + m.ch, mu);
-  load8f(rstd + m.ch, rs);
+  if (rstd) {
+    load8f(rstd + m.ch, rs);
+  } else {
+    load8f(var + m.ch, rs);
+#pragma unroll
+    for (int k = 0; k < 8; ++k) rs[k] = rsqrtf(rs[k] + eps);
+  }
   load8f(gamma + m.ch, ga);
   load8f(beta + m.ch, be);
   for (long long r0 = m.row; r0 < M; r0 += BN_UNROLL * (long long)m.rows) {
@@ -608,7 +614,7 @@ int nb_bn_split(long long M) {
   long long s = ceil_div_ll(M, BN_UNROLL);
   return (int)(s < 1 ? 1 : (s > 592 ? 592 : s));
 }
-// partials: 2 * nb_bn_split(M) * C floats
+// partials: 2 * nb_bn_split(M) * C floats.  rstd null (not in training): from run_var
 int nb_bn_fwd(const void* x, const float* gamma, const float* beta, const void* residual, void* y, float* mean, float* rstd,
               float* run_mean, float* run_var, float* partials, long long M, int C, float eps, float momentum, int relu,
               int training, void* stream) {
@@ -624,7 +630,7 @@ int nb_bn_fwd(const void* x, const float* gamma, const float* beta, const void* 
                                                           run_var);
     NB_LAUNCH_CHECK();
   }
-  bn_apply_kernel<<<bn_grid(M, C, 1 << 20), 256, 0, s>>>((const __nv_bfloat16*)x, mean, rstd, gamma, beta,
+  bn_apply_kernel<<<bn_grid(M, C, 1 << 20), 256, 0, s>>>((const __nv_bfloat16*)x, mean, rstd, run_var, eps, gamma, beta,
                                                         (const __nv_bfloat16*)residual, (__nv_bfloat16*)y, M, C, relu);
   NB_LAUNCH_CHECK();
   return NB_OK;

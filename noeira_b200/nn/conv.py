@@ -13,7 +13,9 @@ import os
 import torch
 
 from .. import ops
-from .._native import check, cuda_lib, ptr, stream_ptr
+from .._native import check, cuda_lib, ptr, raw_stream, stream_ptr
+from ..ops.gemm import ACT, _workspace
+from ..ops.status import status_ptr
 from .init import Constant, Kaiming, Zero
 from .layers import colsum_into
 from .module import Module
@@ -169,25 +171,21 @@ class Conv2D(Module):
         return self.k == 1 and self.stride == 1 and self.pad == 0
 
     def _conv(self, x, w, y, oc, stride, pad, mirror, bias=None, act=None):
-        from ..ops.gemm import ACT, default_workspace
-        from ..ops.status import device_status
         B, H, W, C = x.shape
-        ws = default_workspace(x.device)
-        check(cuda_lib().nb_conv_gemm(ptr(x), ptr(w), ptr(y), *(ctypes.c_int(v) for v in (
-            B, H, W, C, oc, self.k, self.k, stride, pad, int(mirror), w.stride(0), y.stride(0))), ptr(bias), ctypes.c_int(ACT[act]),
-            ptr(device_status(x.device)), ptr(ws), ctypes.c_longlong(ws.numel()), stream_ptr()), "conv_gemm")
+        ws = _workspace(x)
+        check(cuda_lib().nb_conv_gemm(x.data_ptr(), w.data_ptr(), y.data_ptr(), B, H, W, C, oc, self.k, self.k, stride, pad, int(mirror),
+                                      w.stride(0), y.stride(0), None if bias is None else bias.data_ptr(), ACT[act],
+                                      status_ptr(x.get_device()), ws.data_ptr(), ws.numel(), raw_stream()), "conv_gemm")
 
     def _implicit_wgrad(self, d2, B, H, W):
         """dW += patches(x)ᵀ · dy with the patches gathered from the saved NHWC input."""
-        from ..ops.gemm import default_workspace
-        from ..ops.status import device_status
         x, g = self._xin, self.weight.grad_storage
         if (d2.stride(0) * 2) % 16 or d2.data_ptr() % 16:
             d2 = d2.contiguous()
-        ws = default_workspace(x.device)
-        check(cuda_lib().nb_conv_gemm_wgrad(ptr(x), ptr(d2), ptr(g), *(ctypes.c_int(v) for v in (
-            B, H, W, self.icp, self.oc, self.k, self.k, self.stride, self.pad, d2.stride(0), g.stride(0))), ptr(device_status(x.device)),
-            ptr(ws), ctypes.c_longlong(ws.numel()), stream_ptr()), "conv_gemm_wgrad")
+        ws = _workspace(x)
+        check(cuda_lib().nb_conv_gemm_wgrad(x.data_ptr(), d2.data_ptr(), g.data_ptr(), B, H, W, self.icp, self.oc, self.k, self.k,
+                                            self.stride, self.pad, d2.stride(0), g.stride(0), status_ptr(x.get_device()), ws.data_ptr(),
+                                            ws.numel(), raw_stream()), "conv_gemm_wgrad")
 
     def _implicit_dgrad_ok(self, W):
         """Stride-1 layers whose output channels fill 64-wide k-blocks: the input gradient is itself a stride-1 convolution of
@@ -242,15 +240,16 @@ class BatchNorm2D(Module):
         self._x = xc
         y = torch.empty_like(xc)
         self._mean = torch.empty(self.c, device=x.device) if self.training else self.running_mean.data
-        self._rstdv = torch.empty(self.c, device=x.device) if self.training else torch.rsqrt(self.running_var.data + self.eps)
+        # inference: the kernel takes the running variance itself; a backward pass makes its rstd when it comes
+        self._rstdv = torch.empty(self.c, device=x.device) if self.training else None
         lib = cuda_lib()
         split = lib.nb_bn_split(ctypes.c_longlong(M))
         rc = residual.contiguous() if residual is not None else None
-        check(lib.nb_bn_fwd(ptr(xc), ptr(self.gamma.storage), ptr(self.beta.storage), ptr(rc), ptr(y), ptr(self._mean),
-                            ptr(self._rstdv), ptr(self.running_mean.data), ptr(self.running_var.data),
-                            ptr(_scratch(x.device, 2 * split * self.c)), ctypes.c_longlong(M), ctypes.c_int(self.c),
-                            ctypes.c_float(self.eps), ctypes.c_float(self.momentum), ctypes.c_int(int(self.relu)),
-                            ctypes.c_int(int(self.training)), stream_ptr()), "bn_fwd")
+        check(lib.nb_bn_fwd(xc.data_ptr(), self.gamma.storage.data_ptr(), self.beta.storage.data_ptr(), None if rc is None else rc.data_ptr(),
+                            y.data_ptr(), self._mean.data_ptr(), self._rstdv.data_ptr() if self.training else None,
+                            self.running_mean.data.data_ptr(), self.running_var.data.data_ptr(),
+                            _scratch(x.device, 2 * split * self.c).data_ptr(), M, self.c, self.eps, self.momentum, int(self.relu),
+                            int(self.training), raw_stream()), "bn_fwd")
         self._y = y
         return y
 
@@ -271,6 +270,8 @@ class BatchNorm2D(Module):
         d = dy if (dy.is_contiguous() and dy.dtype == torch.bfloat16) else dy.to(torch.bfloat16).contiguous()
         dx = torch.empty_like(d)
         dres = torch.empty_like(d) if self._has_res else None
+        if self._rstdv is None:
+            self._rstdv = torch.rsqrt(self.running_var.data + self.eps)
         lib = cuda_lib()
         split = lib.nb_bn_split(ctypes.c_longlong(M))
         ws = _scratch(dy.device, 2 * split * self.c + 2 * self.c)

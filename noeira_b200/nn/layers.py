@@ -12,7 +12,7 @@ import ctypes
 import torch
 
 from .. import ops
-from .._native import check, cuda_lib, ptr, stream_ptr
+from .._native import check, cuda_lib, ptr, raw_stream, stream_ptr
 from .init import Constant, Initializer, Kaiming, Zero
 from .module import Module
 
@@ -48,9 +48,7 @@ def act_backward(dy, saved, act):
         dy = dy.contiguous()
         saved = saved.contiguous()
         dx = torch.empty_like(dy)
-        check(cuda_lib().nb_act_bwd(ptr(dy), ptr(saved), ptr(dx), ctypes.c_longlong(dy.numel()),
-                                    ctypes.c_int(_act_code(act)),
-                                    stream_ptr()), "act_bwd")
+        check(cuda_lib().nb_act_bwd(dy.data_ptr(), saved.data_ptr(), dx.data_ptr(), dy.numel(), _act_code(act), raw_stream()), "act_bwd")
         return dx
     return dy * act_derivative_cpu(act, saved)
 

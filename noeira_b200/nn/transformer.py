@@ -12,7 +12,7 @@ import math
 import torch
 
 from .. import ops
-from .._native import check, cuda_lib, ptr, stream_ptr
+from .._native import check, cuda_lib, ptr, raw_stream, stream_ptr
 from ..ops.attention import attention_reference, flash_attention_backward, flash_attention_forward
 from .init import Constant, Normal, Zero
 from .layers import Linear
@@ -60,10 +60,9 @@ class _Norm(Module):
         self._x = x2
         y = torch.empty(x2.shape[0], self.dim, device=x.device, dtype=torch.bfloat16)
         self._stats = torch.empty(x2.shape[0], 2, device=x.device, dtype=torch.float32)
-        check(cuda_lib().nb_norm_fwd(ptr(x2), ctypes.c_int(x2.stride(0)), ptr(self.gamma.storage if self.gamma else None),
-                                     ptr(self.beta.storage if self.beta else None), ptr(y), ctypes.c_int(self.dim),
-                                     ptr(self._stats), ctypes.c_int(x2.shape[0]), ctypes.c_int(self.dim),
-                                     ctypes.c_float(self.eps), ctypes.c_int(int(self.RMS)), stream_ptr()), "norm_fwd")
+        check(cuda_lib().nb_norm_fwd(x2.data_ptr(), x2.stride(0), self.gamma.storage.data_ptr() if self.gamma else None,
+                                     self.beta.storage.data_ptr() if self.beta else None, y.data_ptr(), self.dim,
+                                     self._stats.data_ptr(), x2.shape[0], self.dim, self.eps, int(self.RMS), raw_stream()), "norm_fwd")
         return y.reshape(self._shape)
 
     def vjp(self, dy):

@@ -6,8 +6,8 @@ import math
 
 import torch
 
-from .._native import check, cuda_lib, ptr, stream_ptr
-from .status import device_status
+from .._native import check, cuda_lib, ptr, raw_stream, stream_ptr
+from .status import device_status, status_ptr
 
 MASK = {None: 0, "none": 0, "causal": 1, "block_causal": 2}
 
@@ -78,14 +78,11 @@ def flash_attention_forward(q, k, v, scale=None, mask=None, frame=0, causal_off=
     if bias is not None:
         bias = bias.float().contiguous()
         assert bias.shape == (Sq, Sk)
+    addr = lambda t: None if t is None else t.data_ptr()
+    qs, ks, vs = q.stride(), k.stride(), v.stride()
     check(cuda_lib().nb_flash_attn_fwd(
-        ptr(q), ptr(k), ptr(v), ptr(out), ptr(lse), ctypes.c_int(B), ctypes.c_int(Hq), ctypes.c_int(Hkv),
-        ctypes.c_int(Sq), ctypes.c_int(Sk), ctypes.c_int(D),
-        ctypes.c_longlong(q.stride(0)), ctypes.c_longlong(q.stride(1)), ctypes.c_longlong(q.stride(2)),
-        ctypes.c_longlong(k.stride(0)), ctypes.c_longlong(k.stride(1)), ctypes.c_longlong(k.stride(2)),
-        ctypes.c_longlong(v.stride(0)), ctypes.c_longlong(v.stride(1)), ctypes.c_longlong(v.stride(2)),
-        ctypes.c_longlong(out.stride(1)), ctypes.c_float(scale), ctypes.c_int(MASK[mask]), ctypes.c_int(frame),
-        ctypes.c_int(causal_off), ptr(kv), ptr(bias), ptr(device_status(q.device)), stream_ptr()), "flash_attn_fwd")
+        q.data_ptr(), k.data_ptr(), v.data_ptr(), out.data_ptr(), addr(lse), B, Hq, Hkv, Sq, Sk, D, *qs[:3], *ks[:3], *vs[:3], out.stride(1),
+        scale, MASK[mask], frame, causal_off, addr(kv), addr(bias), status_ptr(q.get_device()), raw_stream()), "flash_attn_fwd")
     return out, lse
 
 

@@ -5,9 +5,9 @@ import ctypes
 
 import torch
 
-from .._native import check, cuda_lib, ptr, stream_ptr
-from .status import device_status
-from .streams import ws_key
+from .._native import check, cuda_lib, raw_stream
+from .status import status_ptr
+from .streams import slot, ws_key
 
 ACT = {None: 0, "none": 0, "relu": 1, "tanh": 2, "gelu": 3, "silu": 4, "sigmoid": 5, "add": 16}
 
@@ -31,6 +31,11 @@ def default_workspace(device) -> torch.Tensor:
         w = new_workspace(device)
         _WS[key] = w
     return w
+
+
+def _workspace(t: torch.Tensor) -> torch.Tensor:
+    w = _WS.get((t.get_device(), slot()))
+    return w if w is not None else default_workspace(t.device)
 
 
 TWO_CTA_AUTO, TWO_CTA_OFF, TWO_CTA_FORCE = 0, 1, 2
@@ -58,10 +63,13 @@ def gemm(a: torch.Tensor, b: torch.Tensor, *, a_mn: bool = False, b_mn: bool = F
     if residual is not None:
         assert dact is None and aux is None
         aux, dact = residual, "add"
-    tf32 = a.dtype == torch.float32
-    assert a.dtype == b.dtype and a.dtype in (torch.bfloat16, torch.float32)
-    assert a.stride(-1) == 1 and b.stride(-1) == 1
-    if tf32 and out is None and out_dtype == torch.bfloat16:
+    dt = a.dtype
+    tf32 = dt is torch.float32
+    assert dt is b.dtype and (tf32 or dt is torch.bfloat16)
+    lda, sa = a.stride()
+    ldb, sb = b.stride()
+    assert sa == 1 and sb == 1
+    if tf32 and out is None and out_dtype is torch.bfloat16:
         out_dtype = torch.float32
     if a_mn:
         K, M = a.shape
@@ -76,21 +84,21 @@ def gemm(a: torch.Tensor, b: torch.Tensor, *, a_mn: bool = False, b_mn: bool = F
         N = n
     if out is None:
         out = torch.empty(M, N, device=a.device, dtype=out_dtype)
-    assert out.stride(-1) == 1 and out.shape[0] == M
-    out_f32 = out.dtype == torch.float32
-    assert out_f32 or out.dtype == torch.bfloat16
+    ldd, sd = out.stride()
+    assert sd == 1 and out.shape[0] == M
+    out_f32 = out.dtype is torch.float32
+    assert out_f32 or out.dtype is torch.bfloat16
     if bias is not None:
-        assert bias.dtype == torch.float32 and bias.numel() >= N
+        assert bias.dtype is torch.float32 and bias.numel() >= N
+        bias = bias.data_ptr()
+    ld_aux = 0
     if aux is not None:
-        assert aux.dtype == torch.bfloat16 and aux.stride(-1) == 1
-    st = device_status(a.device)
-    ws = workspace if workspace is not None else default_workspace(a.device)
-    rc = (cuda_lib().nb_gemm_tf32 if tf32 else cuda_lib().nb_gemm_bf16)(
-        ptr(a), ptr(b), ptr(out), ctypes.c_int(M), ctypes.c_int(N), ctypes.c_int(K),
-        ctypes.c_int(a.stride(0)), ctypes.c_int(b.stride(0)), ctypes.c_int(out.stride(0)),
-        ctypes.c_int(int(a_mn)), ctypes.c_int(int(b_mn)), ctypes.c_int(int(out_f32)), ctypes.c_int(int(accumulate)),
-        ctypes.c_float(alpha), ptr(bias), ctypes.c_int(ACT[act]), ptr(aux),
-        ctypes.c_int(aux.stride(0) if aux is not None else 0), ctypes.c_int(ACT[dact]), ptr(st), ctypes.c_int(bn),
-        ptr(ws), ctypes.c_longlong(ws.numel()), stream_ptr())
+        assert aux.dtype is torch.bfloat16 and aux.stride(-1) == 1
+        aux, ld_aux = aux.data_ptr(), aux.stride(0)
+    ws = workspace if workspace is not None else _workspace(a)
+    lib = cuda_lib()
+    rc = (lib.nb_gemm_tf32 if tf32 else lib.nb_gemm_bf16)(
+        a.data_ptr(), b.data_ptr(), out.data_ptr(), M, N, K, lda, ldb, ldd, int(a_mn), int(b_mn), int(out_f32), int(accumulate), alpha,
+        bias, ACT[act], aux, ld_aux, ACT[dact], status_ptr(a.get_device()), bn, ws.data_ptr(), ws.numel(), raw_stream())
     check(rc, "nb_gemm_tf32" if tf32 else "nb_gemm_bf16")
     return out

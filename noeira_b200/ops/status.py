@@ -31,6 +31,17 @@ def device_status(device=None) -> torch.Tensor:
     return t
 
 
+_STATUS_PTR = {}
+
+
+def status_ptr(index: int) -> int:
+    """Address of the status word of CUDA device ``index`` (it lives as long as the process)."""
+    a = _STATUS_PTR.get(index)
+    if a is None:
+        a = _STATUS_PTR[index] = device_status(torch.device("cuda", index)).data_ptr()
+    return a
+
+
 def check_status(device=None, clear: bool = True) -> None:
     t = device_status(device)
     code, where, block, extra = (int(x) for x in t.cpu())

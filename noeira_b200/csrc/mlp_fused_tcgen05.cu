@@ -56,6 +56,24 @@ struct MlpGroup {
   MlpParams prm[2];
 };
 
+// One warp's part (32 rows x 128 columns = two k-blocks) of a [128 x 256] bf16 tile in the swizzled K-major layout, from shared
+// to global memory in runs of 128 bytes.  Stored by the lane that owns the row, a warp instruction touched 32 rows with 16
+// bytes each, in front of the barrier that the next layer waits for.  16384 rows, two networks: forward 38 us -> 23,
+// backward 35 us -> 32 (with the biases out of the loop and the third W2 k-block ahead of time).
+__device__ __forceinline__ void copy_tile_out(const uint8_t* tile, __nv_bfloat16* dst, int ld, int row0, int M, int quarter, int half,
+                                              int lane) {
+#pragma unroll
+  for (int kbi = 0; kbi < 2; ++kbi) {
+    const int kb = half * 2 + kbi, ch = lane & 7;
+#pragma unroll
+    for (int i = 0; i < 8; ++i) {
+      const int rr = quarter * 32 + i * 4 + (lane >> 3);
+      const uint4 v = *reinterpret_cast<const uint4*>(tile + kb * 16384 + (rr >> 3) * 1024 + (rr & 7) * 128 + ((ch ^ (rr & 7)) << 4));
+      if (row0 + rr < M) *reinterpret_cast<uint4*>(dst + (size_t)(row0 + rr) * ld + kb * 64 + ch * 8) = v;
+    }
+  }
+}
+
 // blockIdx.y selects the network: the actor and the critic of an RL update run in ONE launch.
 __global__ void __launch_bounds__(MLP_THREADS, 1)
 mlp3_fwd_kernel(const __grid_constant__ MlpGroup grp) {
@@ -80,8 +98,8 @@ mlp3_fwd_kernel(const __grid_constant__ MlpGroup grp) {
   uint8_t* sW3 = sH + H_BYTES;
   uint64_t* bars = reinterpret_cast<uint64_t*>(sW3 + W3_BYTES);
   uint64_t* x_full = bars;
-  uint64_t* w2_full = bars + 1;    // [2]
-  uint64_t* w2_empty = bars + 3;   // [2]
+  uint64_t* w2_full = bars + 1;    // [3]: two stages, and W1's memory once layer 1 has read it
+  uint64_t* w2_empty = bars + 4;   // of stage 0
   uint64_t* acc_full = bars + 5;   // [3]
   uint64_t* h_ready = bars + 8;    // [2]
   uint64_t* w3_ready = bars + 10;
@@ -93,12 +111,12 @@ mlp3_fwd_kernel(const __grid_constant__ MlpGroup grp) {
 
   if (threadIdx.x == 0) {
     mbar_init(x_full, 1);
-    for (int i = 0; i < 2; ++i) {
+    mbar_init(w2_empty, 1);
+    for (int i = 0; i < 2; ++i) mbar_init(&h_ready[i], 8);
+    for (int i = 0; i < 3; ++i) {
+      mbar_init(&acc_full[i], 1);
       mbar_init(&w2_full[i], 1);
-      mbar_init(&w2_empty[i], 1);
-      mbar_init(&h_ready[i], 8);
     }
-    for (int i = 0; i < 3; ++i) mbar_init(&acc_full[i], 1);
     mbar_init(w3_ready, 8);
     *abort_flag = 0;
     fence_barrier_init();
@@ -120,11 +138,13 @@ mlp3_fwd_kernel(const __grid_constant__ MlpGroup grp) {
       mbar_expect_tx(x_full, X_BYTES + W1_BYTES);
       tma_load_2d(sX, &tmX, x_full, 0, row0);                                   // box {64 k, 128 rows}, zero fill past k0 / M
       for (int h = 0; h < HID / 64; ++h) tma_load_2d(sW1 + h * 8192, &tmW1, x_full, h * 64, 0);   // boxes {64 n, 64 k}
+      // k-blocks 0 and 1 at once, 2 into W1's memory as soon as layer 1 is through, 3 into stage 0 when block 0 is used up
       for (int kb = 0; kb < HID / 64; ++kb) {
-        const int st = kb & 1;
-        if (*abort_flag || !mbar_wait(&w2_empty[st], ((uint32_t)(kb >> 1) & 1u) ^ 1u, p.status, 301)) { *abort_flag = 1; break; }
+        const int st = kb == 3 ? 0 : kb;
+        if (kb >= 2 && (*abort_flag || !mbar_wait(kb == 2 ? &acc_full[0] : w2_empty, 0u, p.status, 301))) { *abort_flag = 1; break; }
+        uint8_t* dst = st == 2 ? sW1 : sW2 + st * W2_STAGE;
         mbar_expect_tx(&w2_full[st], W2_STAGE);
-        for (int h = 0; h < HID / 64; ++h) tma_load_2d(sW2 + st * W2_STAGE + h * 8192, &tmW2, &w2_full[st], h * 64, kb * 64);
+        for (int h = 0; h < HID / 64; ++h) tma_load_2d(dst + h * 8192, &tmW2, &w2_full[st], h * 64, kb * 64);
       }
     }
   } else if (warp == 1) {
@@ -143,15 +163,15 @@ mlp3_fwd_kernel(const __grid_constant__ MlpGroup grp) {
       }
       if (ok) ok = mbar_wait(&h_ready[0], 0u, p.status, 311);
       for (int kb = 0; kb < HID / 64 && ok; ++kb) {
-        const int st = kb & 1;
-        if (!mbar_wait(&w2_full[st], (uint32_t)(kb >> 1) & 1u, p.status, 312)) { ok = false; break; }
+        const int st = kb == 3 ? 0 : kb;
+        if (!mbar_wait(&w2_full[st], kb == 3 ? 1u : 0u, p.status, 312)) { ok = false; break; }
         tc_fence_after();
-        const uint32_t ha = smem_u32(sH + kb * 16384), wb = smem_u32(sW2 + st * W2_STAGE);
+        const uint32_t ha = smem_u32(sH + kb * 16384), wb = smem_u32(st == 2 ? sW1 : sW2 + st * W2_STAGE);
 #pragma unroll
         for (int k = 0; k < 4; ++k)
           umma_f16(tmem_base + 256, make_smem_desc(ha + k * 32, 16, 1024, 2),
                    make_smem_desc(wb + k * (16 * 128), 8192, 1024, 2), idesc_h, (kb | k) != 0 ? 1u : 0u);
-        umma_commit(&w2_empty[st]);
+        if (kb == 0) umma_commit(w2_empty);
       }
       if (ok) umma_commit(&acc_full[1]);
       if (ok) ok = mbar_wait(&h_ready[1], 0u, p.status, 313) && mbar_wait(w3_ready, 0u, p.status, 314);
@@ -176,13 +196,21 @@ mlp3_fwd_kernel(const __grid_constant__ MlpGroup grp) {
     const int t = (warp - 2) * 32 + lane;         // 0..255 for cooperative loads
     const uint32_t lane_addr = tmem_base + ((uint32_t)(quarter * 32) << 16);
     // ---- stage W3ᵀ: element (n, k) of the K-major [16 x 256] tile
-    for (int e = t; e < N3P * HID; e += EPI_THREADS) {
-      const int k = e / N3P, n = e - k * N3P;
-      const __nv_bfloat16 v = (n < p.n3) ? p.w3[(size_t)k * p.ld_w3 + n] : __float2bfloat16(0.f);
-      const int kb = k >> 6, kk = k & 63;
-      uint8_t* dst = sW3 + kb * 2048 + (n >> 3) * 1024 + (n & 7) * 128 + ((((kk >> 3) ^ (n & 7))) << 4) + (kk & 7) * 2;
-      *reinterpret_cast<__nv_bfloat16*>(dst) = v;
+    // (thread = row k; its up to 16 loads are in flight together)
+    {
+      const int k = t, kb = k >> 6, kk = k & 63;
+      __nv_bfloat16 v[N3P];
+#pragma unroll
+      for (int n = 0; n < N3P; ++n) v[n] = n < p.n3 ? p.w3[(size_t)k * p.ld_w3 + n] : __float2bfloat16(0.f);
+#pragma unroll
+      for (int n = 0; n < N3P; ++n)
+        *reinterpret_cast<__nv_bfloat16*>(sW3 + kb * 2048 + (n >> 3) * 1024 + (n & 7) * 128 + ((((kk >> 3) ^ (n & 7))) << 4) + (kk & 7) * 2) = v[n];
     }
+    // the biases of this warp's 128 columns, four per lane, out of the loops below
+    const int c4 = half * 128 + 4 * lane;
+    const float4 zf = make_float4(0.f, 0.f, 0.f, 0.f);
+    const float4 bias1 = p.b1 ? __ldg(reinterpret_cast<const float4*>(p.b1 + c4)) : zf;
+    const float4 bias2 = p.b2 ? __ldg(reinterpret_cast<const float4*>(p.b2 + c4)) : zf;
     fence_proxy_async();
     __syncwarp();
     if (lane == 0) mbar_arrive(w3_ready);
@@ -191,7 +219,7 @@ mlp3_fwd_kernel(const __grid_constant__ MlpGroup grp) {
     for (int layer = 0; layer < 2 && ok; ++layer) {
       if (!__all_sync(0xffffffffu, !*abort_flag && mbar_wait(&acc_full[layer], 0u, p.status, 320 + layer))) { ok = false; break; }
       tc_fence_after();
-      const float* bias = layer == 0 ? p.b1 : p.b2;
+      const float4 bias = layer == 0 ? bias1 : bias2;
       __nv_bfloat16* hsave = layer == 0 ? p.h1 : p.h2;
       const uint32_t acc = lane_addr + (uint32_t)(layer * 256 + half * 128);
       // 32 columns per step, two register sets in ping-pong: the next step's TMEM load is in flight while this one is
@@ -201,7 +229,9 @@ mlp3_fwd_kernel(const __grid_constant__ MlpGroup grp) {
         uint32_t pk[16];
 #pragma unroll
         for (int j = 0; j < 32; j += 4) {
-          const float4 bv = bias ? __ldg(reinterpret_cast<const float4*>(bias + c0 + j)) : make_float4(0.f, 0.f, 0.f, 0.f);
+          const int bl = s4 * 8 + j / 4;
+          const float4 bv = make_float4(__shfl_sync(0xffffffffu, bias.x, bl), __shfl_sync(0xffffffffu, bias.y, bl),
+                                        __shfl_sync(0xffffffffu, bias.z, bl), __shfl_sync(0xffffffffu, bias.w, bl));
           __nv_bfloat162 a = __floats2bfloat162_rn(act1(p.act, __uint_as_float(cur[j]) + bv.x),
                                                    act1(p.act, __uint_as_float(cur[j + 1]) + bv.y));
           __nv_bfloat162 b = __floats2bfloat162_rn(act1(p.act, __uint_as_float(cur[j + 2]) + bv.z),
@@ -215,11 +245,6 @@ mlp3_fwd_kernel(const __grid_constant__ MlpGroup grp) {
 #pragma unroll
         for (int q = 0; q < 4; ++q)
           *reinterpret_cast<uint4*>(base + (((ch + q) ^ (r & 7)) << 4)) = make_uint4(pk[4 * q], pk[4 * q + 1], pk[4 * q + 2], pk[4 * q + 3]);
-        if (hsave && row < p.M) {
-          uint4* g = reinterpret_cast<uint4*>(hsave + (size_t)row * p.ld_h + c0);
-#pragma unroll
-          for (int q = 0; q < 4; ++q) g[q] = make_uint4(pk[4 * q], pk[4 * q + 1], pk[4 * q + 2], pk[4 * q + 3]);
-        }
       };
       uint32_t ra[32], rb[32];
       tmem_ld_32x32b_x32_nowait(acc, ra);
@@ -238,6 +263,8 @@ mlp3_fwd_kernel(const __grid_constant__ MlpGroup grp) {
       fence_proxy_async();
       __syncwarp();
       if (lane == 0) mbar_arrive(&h_ready[layer]);
+      // the saved activations leave from shared memory while the tensor core works on the next layer
+      if (hsave) copy_tile_out(sH, hsave, p.ld_h, row0, p.M, quarter, half, lane);
     }
     if (ok && !__all_sync(0xffffffffu, !*abort_flag && mbar_wait(&acc_full[2], 0u, p.status, 322))) ok = false;
     if (ok && half == 0) {
@@ -343,8 +370,8 @@ mlp3_bwd_kernel(const __grid_constant__ MlpBwdGroup grp) {
   uint8_t* sW2 = sW3 + W3_BYTES;            // 2 stages
   uint8_t* sG = sW2 + 2 * W2_STAGE;
   uint64_t* bars = reinterpret_cast<uint64_t*>(sG + G_BYTES);
-  uint64_t* w2_full = bars;        // [2]
-  uint64_t* w2_empty = bars + 2;   // [2]
+  uint64_t* w2_full = bars;        // [3]: two stages, and W3's memory once the first product has read it
+  uint64_t* w2_empty = bars + 3;   // of stage 0
   uint64_t* acc_full = bars + 4;   // [2]
   uint64_t* staged = bars + 6;     // dY and W3 tiles written (4 warps)
   uint64_t* g_ready = bars + 7;    // G2 tile written (4 warps)
@@ -354,11 +381,9 @@ mlp3_bwd_kernel(const __grid_constant__ MlpBwdGroup grp) {
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int row0 = blockIdx.x * ROWS;
   if (threadIdx.x == 0) {
-    for (int i = 0; i < 2; ++i) {
-      mbar_init(&w2_full[i], 1);
-      mbar_init(&w2_empty[i], 1);
-      mbar_init(&acc_full[i], 1);
-    }
+    for (int i = 0; i < 3; ++i) mbar_init(&w2_full[i], 1);
+    for (int i = 0; i < 2; ++i) mbar_init(&acc_full[i], 1);
+    mbar_init(w2_empty, 1);
     mbar_init(staged, 8);
     mbar_init(g_ready, 8);
     *abort_flag = 0;
@@ -377,11 +402,11 @@ mlp3_bwd_kernel(const __grid_constant__ MlpBwdGroup grp) {
   if (warp == 0) {
     if (elect_one()) {
       for (int kb = 0; kb < HID / 64; ++kb) {
-        const int st = kb & 1;
-        if (*abort_flag || !mbar_wait(&w2_empty[st], ((uint32_t)(kb >> 1) & 1u) ^ 1u, p.status, 331)) { *abort_flag = 1; break; }
+        const int st = kb == 3 ? 0 : kb;
+        if (kb >= 2 && (*abort_flag || !mbar_wait(kb == 2 ? &acc_full[0] : w2_empty, 0u, p.status, 331))) { *abort_flag = 1; break; }
         mbar_expect_tx(&w2_full[st], W2_STAGE);
         // B(n, k) of G2 W2ᵀ is W2[n, k]: row n of the [IN, OUT] matrix, 64 consecutive columns
-        tma_load_2d(sW2 + st * W2_STAGE, &tmW2, &w2_full[st], kb * 64, 0);
+        tma_load_2d(st == 2 ? sW3 : sW2 + st * W2_STAGE, &tmW2, &w2_full[st], kb * 64, 0);
       }
     }
   } else if (warp == 1) {
@@ -395,15 +420,15 @@ mlp3_bwd_kernel(const __grid_constant__ MlpBwdGroup grp) {
         ok = mbar_wait(g_ready, 0u, p.status, 341);
       }
       for (int kb = 0; kb < HID / 64 && ok; ++kb) {
-        const int st = kb & 1;
-        if (!mbar_wait(&w2_full[st], (uint32_t)(kb >> 1) & 1u, p.status, 342)) { ok = false; break; }
+        const int st = kb == 3 ? 0 : kb;
+        if (!mbar_wait(&w2_full[st], kb == 3 ? 1u : 0u, p.status, 342)) { ok = false; break; }
         tc_fence_after();
-        const uint32_t ga = smem_u32(sG + kb * 16384), wb = smem_u32(sW2 + st * W2_STAGE);
+        const uint32_t ga = smem_u32(sG + kb * 16384), wb = smem_u32(st == 2 ? sW3 : sW2 + st * W2_STAGE);
 #pragma unroll
         for (int k = 0; k < 4; ++k)
           umma_f16(tmem_base + 256, make_smem_desc(ga + k * 32, 16, 1024, 2), make_smem_desc(wb + k * 32, 16, 1024, 2), idesc,
                    (kb | k) != 0 ? 1u : 0u);
-        umma_commit(&w2_empty[st]);
+        if (kb == 0) umma_commit(w2_empty);
       }
       if (ok) umma_commit(&acc_full[1]);
       if (!ok) *abort_flag = 1;
@@ -454,10 +479,7 @@ mlp3_bwd_kernel(const __grid_constant__ MlpBwdGroup grp) {
     bool ok = true;
     uint8_t* grow = sG + (r >> 3) * 1024 + (r & 7) * 128;
     for (int layer = 0; layer < 2 && ok; ++layer) {
-      if (!__all_sync(0xffffffffu, !*abort_flag && mbar_wait(&acc_full[layer], 0u, p.status, 350 + layer))) { ok = false; break; }
-      tc_fence_after();
       const __nv_bfloat16* hsrc = (layer == 0 ? p.h2 : p.h1) + (size_t)row * p.ld_h;
-      __nv_bfloat16* gdst = (layer == 0 ? p.g2 : p.g1) + (size_t)row * p.ld_g;
       const uint32_t acc = lane_addr + (uint32_t)(layer * 256 + half * 128);
       auto process = [&](const uint32_t (&cur)[32], const uint4 (&hv)[4], int s4) {
         const int c0 = half * 128 + s4 * 32;
@@ -470,20 +492,13 @@ mlp3_bwd_kernel(const __grid_constant__ MlpBwdGroup grp) {
                                                    __uint_as_float(cur[2 * j + 1]) * dact1(p.act, h1));
           pk[j] = *reinterpret_cast<uint32_t*>(&g);
         }
-        if (layer == 0 || part) {
-          // layer 0: G2 is the A operand of the second product.  layer 1: that product has completed (acc_full[1]),
-          // so the same tile holds G1 for the column sums.
-          const int kb = c0 >> 6, ch = (c0 & 63) >> 3;
-          uint8_t* base = grow + kb * 16384;
+        // layer 0: G2 is the A operand of the second product.  layer 1: that product has completed (acc_full[1]), so the
+        // same tile holds G1 for the column sums and the way out.
+        const int kb = c0 >> 6, ch = (c0 & 63) >> 3;
+        uint8_t* base = grow + kb * 16384;
 #pragma unroll
-          for (int q = 0; q < 4; ++q)
-            *reinterpret_cast<uint4*>(base + (((ch + q) ^ (r & 7)) << 4)) = make_uint4(pk[4 * q], pk[4 * q + 1], pk[4 * q + 2], pk[4 * q + 3]);
-        }
-        if (row < p.M) {
-          uint4* g = reinterpret_cast<uint4*>(gdst + c0);
-#pragma unroll
-          for (int q = 0; q < 4; ++q) g[q] = make_uint4(pk[4 * q], pk[4 * q + 1], pk[4 * q + 2], pk[4 * q + 3]);
-        }
+        for (int q = 0; q < 4; ++q)
+          *reinterpret_cast<uint4*>(base + (((ch + q) ^ (r & 7)) << 4)) = make_uint4(pk[4 * q], pk[4 * q + 1], pk[4 * q + 2], pk[4 * q + 3]);
       };
       auto load_h = [&](uint4 (&hv)[4], int s4) {
 #pragma unroll
@@ -493,11 +508,13 @@ mlp3_bwd_kernel(const __grid_constant__ MlpBwdGroup grp) {
       // two register sets in ping-pong, written out as four steps (no loop-carried register copy before a wait)
       uint32_t ra[32], rb[32];
       uint4 ha[4], hb[4];
+      load_h(ha, 0);          // ahead of the product they are multiplied with
+      load_h(hb, 1);
+      if (!__all_sync(0xffffffffu, !*abort_flag && mbar_wait(&acc_full[layer], 0u, p.status, 350 + layer))) { ok = false; break; }
+      tc_fence_after();
       tmem_ld_32x32b_x32_nowait(acc, ra);
-      load_h(ha, 0);
       tmem_ld_wait();
       tmem_ld_32x32b_x32_nowait(acc + 32u, rb);
-      load_h(hb, 1);
       process(ra, ha, 0);
       tmem_ld_wait();
       tmem_ld_32x32b_x32_nowait(acc + 64u, ra);
@@ -515,6 +532,8 @@ mlp3_bwd_kernel(const __grid_constant__ MlpBwdGroup grp) {
         __syncwarp();
         if (lane == 0) mbar_arrive(g_ready);
       }
+      __syncwarp();
+      copy_tile_out(sG, layer == 0 ? p.g2 : p.g1, p.ld_g, row0, p.M, quarter, half, lane);
       if (part) {
         asm volatile("bar.sync 1, 256;" ::: "memory");   // the whole tile is written
         part[(layer == 0 ? HID : 0) + t] = tile_colsum(sG, t);       // [0] g1, [1] g2, [2] dy

@@ -21,6 +21,7 @@ from .layers import colsum_into
 from .module import Module
 
 _WS = {}
+_WS_KEPT = []
 
 
 def _scratch(device, n):
@@ -28,7 +29,10 @@ def _scratch(device, n):
     key = ws_key(device)
     t = _WS.get(key)
     if t is None or t.numel() < n:
-        t = torch.empty(max(n, 1 << 20), dtype=torch.float32, device=device)
+        # a captured graph may hold the smaller buffer's address: it stays alive, and doubling bounds what is kept
+        if t is not None:
+            _WS_KEPT.append(t)
+        t = torch.empty(max(n, 2 * t.numel() if t is not None else 1 << 20), dtype=torch.float32, device=device)
         _WS[key] = t
     return t
 

@@ -191,7 +191,7 @@ def register_bounds_status(status_tensor) -> int:
     if key in lib._bounds_registered:
         return 0
     n = 0
-    for tu in ("misc_ops", "replay", "ppo_kernels"):
+    for tu in ("misc_ops", "replay", "ppo_kernels", "conv_gemm"):
         fn = getattr(lib, f"nb_bounds_register_{tu}", None)
         if fn is not None:
             check(fn(ctypes.c_void_p(key)), f"bounds_register_{tu}")

@@ -18,12 +18,15 @@
 //     the GEMM (gemm_tile.cuh).
 // Bound by the gather: 1024 16-byte copies per 128 x 64 block and SM, 360 to 410 ns, so wider B tiles come almost free.
 // Counterpart in the reference: im2col + GEMM (noeira/nn/primitives/conv2d.mojo:437,652,723) or cuDNN.
+#include "conv_index.h"
 #include "gemm_tile.cuh"
 
 namespace {
 
 using namespace nb;
 using namespace nbgemm;
+using namespace nbconv;
+static_assert(TILE_ROWS == BM && K_BLOCK == BK, "one tiling for the kernel and its index functions");
 
 // Two groups of four gathering warps take the k-blocks in turn: a k-block costs its warps about 900 clocks, most of them
 // latency (barrier, proxy fence, address arithmetic of one warp per scheduler), and only half of that is left per k-block.
@@ -31,27 +34,6 @@ using namespace nbgemm;
 constexpr int CP_GROUPS = 2, CP_GROUP_WARPS = 4, CP_WARPS = CP_GROUPS * CP_GROUP_WARPS;
 constexpr int CONV_EPI_WARPS = 4;   // enough behind a main loop this long, and leaves 128 registers per thread
 constexpr int CONV_THREADS = 32 * (CP_WARPS + 2 + CONV_EPI_WARPS);   // gather, MMA, B loads, epilogue
-
-// n / d for 0 <= n < 2^31 by one multiplication (Granlund and Montgomery, "Division by invariant integers using
-// multiplication"): with l = ceil(log2 d), m = floor(2^(31 + l) / d) + 1 fits in 32 bits and n / d = (n m) >> (31 + l).
-struct FastDiv {
-  uint32_t mul, shift;   // shift = l − 1 after the high word; d = 1: mul = 0
-  __host__ void set(uint32_t d) {
-    uint32_t l = 0;
-    while ((1ull << l) < d) ++l;
-    mul = d == 1 ? 0u : (uint32_t)((1ull << (31 + l)) / d + 1);
-    shift = d == 1 ? 0u : l - 1;
-  }
-  __device__ __forceinline__ int div(int n) const { return mul ? (int)(__umulhi((uint32_t)n, mul) >> shift) : n; }
-};
-
-struct ConvGeom {
-  const __nv_bfloat16* x;
-  int H, W, C, KW, taps, stride, pad, OH, OW, pixels;   // pixels = B·OH·OW
-  FastDiv by_cv, by_kw, by_image, by_row;               // chunks per tap, taps per filter row, OH·OW, OW
-  int wgrad;    // A = patches^T (MN-major), reduction over the pixels
-  int mirror;   // B rows of tap t are those of tap taps − 1 − t, K-major (data gradient)
-};
 
 __device__ __forceinline__ void cp_async16(uint32_t dst, const void* src, bool valid) {
   asm volatile("cp.async.ca.shared.global [%0], [%1], 16, %2;" ::"r"(dst), "l"(src), "r"(valid ? 16 : 0) : "memory");
@@ -62,41 +44,11 @@ __device__ __forceinline__ void cp_wait() {
   asm volatile("cp.async.wait_group %0;" ::"n"(N) : "memory");
 }
 
-// Output pixel m as its window's corner in the input; a pixel past the last one gets a corner that fails every bound.
-struct Corner { int h, w, off; };   // off: element offset of (h, w, channel 0), may be negative
-struct Pixel { int b, oh, ow; };
-__device__ __forceinline__ Pixel pixel_of(const ConvGeom& g, int m) {
-  const int b = g.by_image.div(m), r = m - b * (g.OH * g.OW), oh = g.by_row.div(r);
-  return Pixel{b, oh, r - oh * g.OW};
-}
-__device__ __forceinline__ void pixel_step(const ConvGeom& g, Pixel& p, int n) {
-  p.ow += n;
-  while (p.ow >= g.OW) {
-    p.ow -= g.OW;
-    if (++p.oh == g.OH) { p.oh = 0; ++p.b; }
-  }
-}
-__device__ __forceinline__ Corner corner_of(const ConvGeom& g, const Pixel& p, int m) {
-  Corner c;
-  c.h = m < g.pixels ? p.oh * g.stride - g.pad : -(1 << 28);
-  c.w = p.ow * g.stride - g.pad;
-  c.off = ((p.b * g.H + p.oh * g.stride - g.pad) * g.W + c.w) * g.C;
-  return c;
-}
-// 16-byte chunk q of a patch: 8 channels of one tap
-struct Tap { int kh, kw, off; };
-__device__ __forceinline__ Tap tap_of(const ConvGeom& g, int q) {
-  const int t = g.by_cv.div(q), c8 = q - t * (g.C >> 3);
-  Tap k;
-  k.kh = g.by_kw.div(t);
-  k.kw = t - k.kh * g.KW;
-  k.off = (k.kh * g.W + k.kw) * g.C + c8 * 8;
-  if (t >= g.taps) k.kh = 1 << 28;                   // fails every bound
-  return k;
-}
 __device__ __forceinline__ void gather(const ConvGeom& g, uint32_t dst, const Corner& c, const Tap& k) {
-  const bool in = (unsigned)(c.h + k.kh) < (unsigned)g.H && (unsigned)(c.w + k.kw) < (unsigned)g.W;
-  cp_async16(dst, g.x + (in ? c.off + k.off : 0), in);
+  int off;
+  bool in = chunk_of(g, c, k, off);
+  if (!NB_IN_BOUNDS(!in || (off >= 0 && off <= g.elems - 8), 641, off)) in = false;
+  cp_async16(dst, (const __nv_bfloat16*)g.x + (in ? off : 0), in);
 }
 
 template <int BN, int STAGES, int MODE>
@@ -378,23 +330,15 @@ int conv_geom(ConvGeom& g, const void* x, int B, int H, int W, int C, int KH, in
   if (B <= 0 || H <= 0 || W <= 0 || C <= 0 || C % 8 || KH <= 0 || KW <= 0 || stride <= 0 || pad < 0) return NB_ERR_BAD_ARG;
   if (H + 2 * pad < KH || W + 2 * pad < KW) return NB_ERR_BAD_ARG;
   if (reinterpret_cast<uintptr_t>(x) & 15) return NB_ERR_UNALIGNED;
-  g.x = (const __nv_bfloat16*)x;
-  g.H = H; g.W = W; g.C = C; g.KW = KW; g.taps = KH * KW; g.stride = stride; g.pad = pad;
-  g.OH = (H + 2 * pad - KH) / stride + 1;
-  g.OW = (W + 2 * pad - KW) / stride + 1;
-  // offsets are 32-bit element counts, with the window's corner up to pad rows and columns outside
-  if (((long long)B * H + 2 * pad) * (W + 2LL * pad) * C > 0x7fffffffLL || (long long)B * g.OH * g.OW > 0x7fffffffLL - 256)
-    return NB_ERR_TOO_LARGE;
-  g.pixels = B * g.OH * g.OW;
-  g.by_cv.set(C / 8);
-  g.by_kw.set(KW);
-  g.by_image.set(g.OH * g.OW);
-  g.by_row.set(g.OW);
-  g.wgrad = g.mirror = 0;
+  if (!conv_fits(B, H, W, C, KH, KW, stride, pad)) return NB_ERR_TOO_LARGE;
+  g.x = x;
+  conv_geom_set(g, B, H, W, C, KH, KW, stride, pad);
   return NB_OK;
 }
 
 }  // namespace
+
+NB_BOUNDS_REGISTER(conv_gemm)
 
 extern "C" {
 

@@ -43,6 +43,14 @@ def main():
         return 1
     except DeviceStatusError as e:
         assert e.code == 3 and e.where == 611 and e.extra == 64
+    # the convolution's gather with pixels and taps past the last one in the same tile: every offset it admits is inside x
+    for ic, oc, k, stride, pad, b, h, w in ((64, 64, 3, 1, 2, 1, 4, 3), (3, 64, 7, 2, 3, 2, 33, 45), (72, 40, 5, 3, 2, 2, 19, 14),
+                                            (64, 64, 3, 1, 1, 2, 17, 23), (8, 8, 3, 1, 0, 1, 5, 4)):
+        conv = nn.Conv2D(ic, oc, k, stride, pad).to("cuda")
+        y = conv.forward(torch.randn(b, h, w, conv.icp, device="cuda").bfloat16())
+        conv.vjp(torch.ones_like(y))
+        torch.cuda.synchronize()
+        check_status()
     # the context is still healthy
     assert float((torch.ones(4, device="cuda") * 2).sum()) == 8.0
     check_status()

@@ -280,6 +280,7 @@ template <int BN, int STAGES>
 int launch_conv(const CUtensorMap& tmB, GemmParams& p, const ConvGeom& g, int splits, cudaStream_t stream) {
   constexpr size_t smem = (size_t)STAGES * (BM * BK * 2 + BN * BK * 2) + CONV_EPI_WARPS * EPI_STAGE_BYTES + 1024 /*align*/ + 256 /*barriers*/;
   static_assert(smem <= 232448, "shared memory budget of one CTA");
+  set_vec(p);
   p.tiles_m = ceil_div(p.M, BM);
   p.tiles_n = ceil_div(p.N, BN);
   p.tile_rows = BM;

@@ -413,12 +413,12 @@ struct EpiPrefetch {
 
 __device__ __forceinline__ void epilogue_prefetch16(const GemmParams& p, int row, int col0, bool active, EpiPrefetch& pf) {
   if (!active || col0 + 16 > p.N) return;
-  if (p.dact && (p.ld_aux % 8 == 0)) {
+  if (p.dact && p.vec_aux) {
     const __nv_bfloat16* ax = p.aux + (size_t)row * p.ld_aux + col0;
     pf.aux[0] = __ldg(reinterpret_cast<const uint4*>(ax));
     pf.aux[1] = __ldg(reinterpret_cast<const uint4*>(ax + 8));
   }
-  if (p.out_f32 && p.accumulate && (p.ldd % 4 == 0)) {
+  if (p.out_f32 && p.accumulate && p.vec_d) {
     const float* o = reinterpret_cast<const float*>(p.D) + (size_t)row * p.ldd + col0;
 #pragma unroll
     for (int j = 0; j < 4; ++j) pf.old[j] = *reinterpret_cast<const float4*>(o + 4 * j);
@@ -431,7 +431,7 @@ __device__ __forceinline__ void epilogue_store16(const GemmParams& p, int row, i
   const bool full = (col0 + 16 <= p.N);
   float sv[16];
   if (p.dact) {
-    if (full && (p.ld_aux % 8 == 0)) {
+    if (full && p.vec_aux) {
       unpack16(pf.aux, sv);
     } else {
       const __nv_bfloat16* ax = p.aux + (size_t)row * p.ld_aux + col0;
@@ -442,7 +442,7 @@ __device__ __forceinline__ void epilogue_store16(const GemmParams& p, int row, i
 #pragma unroll
   for (int j = 0; j < 16; ++j) v[j] *= p.alpha;
   if (p.bias) {
-    if (full) {
+    if (full && p.vec_bias) {
 #pragma unroll
       for (int j = 0; j < 16; j += 4) {
         const float4 bv = __ldg(reinterpret_cast<const float4*>(p.bias + col0 + j));
@@ -458,7 +458,7 @@ __device__ __forceinline__ void epilogue_store16(const GemmParams& p, int row, i
   if (p.dact) dact_apply16(p.dact, v, sv);
   if (p.out_f32) {
     float* o = reinterpret_cast<float*>(p.D) + (size_t)row * p.ldd + col0;
-    if (full && (p.ldd % 4 == 0)) {
+    if (full && p.vec_d) {
 #pragma unroll
       for (int j = 0; j < 16; j += 4) {
         float4 x = make_float4(v[j], v[j + 1], v[j + 2], v[j + 3]);
@@ -475,7 +475,7 @@ __device__ __forceinline__ void epilogue_store16(const GemmParams& p, int row, i
     }
   } else {
     __nv_bfloat16* o = reinterpret_cast<__nv_bfloat16*>(p.D) + (size_t)row * p.ldd + col0;
-    if (full && (p.ldd % 8 == 0)) {
+    if (full && p.vec_d) {
 #pragma unroll
       for (int j = 0; j < 16; j += 8) *reinterpret_cast<uint4*>(o + j) = pack8f(v + j);
     } else {
@@ -567,7 +567,7 @@ splitk_reduce_f32_kernel(const GemmParams p, int BN) {
   }
   v.x *= p.alpha; v.y *= p.alpha; v.z *= p.alpha; v.w *= p.alpha;
   float* o = reinterpret_cast<float*>(p.D) + (size_t)row * p.ldd + col0;
-  if (col0 + 4 <= p.N && (p.ldd % 4 == 0)) {
+  if (col0 + 4 <= p.N && p.vec_d) {
     if (p.accumulate) {
       const float4 y = *reinterpret_cast<const float4*>(o);
       v.x += y.x; v.y += y.y; v.z += y.z; v.w += y.w;
@@ -603,6 +603,7 @@ template <int BN, int STAGES>
 int launch(const CUtensorMap& tmA, const CUtensorMap& tmB, GemmParams& p, int splits, cudaStream_t stream) {
   constexpr size_t smem = (size_t)STAGES * (BM * BK * 2 + BN * BK * 2) + EPI_WARPS * EPI_STAGE_BYTES + 1024 /*align*/ + 256 /*barriers*/;
   static_assert(smem <= 232448, "shared memory budget of one CTA");
+  set_vec(p);
   p.tiles_m = ceil_div(p.M, BM);
   p.tiles_n = ceil_div(p.N, BN);
   p.tile_rows = BM;
@@ -632,6 +633,7 @@ int launch(const CUtensorMap& tmA, const CUtensorMap& tmB, GemmParams& p, int sp
 int launch_two_cta(const CUtensorMap& tmA, const CUtensorMap& tmB, GemmParams& p, int splits, cudaStream_t stream) {
   constexpr size_t smem = (size_t)STAGES2 * (BM * BK * 2 + (BN2 / 2) * BK * 2) + EPI_WARPS * EPI_STAGE_BYTES + 1024 /*align*/ + 256 /*barriers*/;
   static_assert(smem <= 232448, "shared memory budget of one CTA");
+  set_vec(p);
   p.tiles_m = ceil_div(p.M, 2 * BM);
   p.tiles_n = ceil_div(p.N, BN2);
   p.tile_rows = 2 * BM;

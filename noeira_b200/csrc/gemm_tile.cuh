@@ -29,6 +29,7 @@ struct GemmParams {
   int tiles_m, tiles_n, num_kb;
   int splits, kb_per_split;  // split-K: work item = (tile, split); partial tiles meet in `ws`
   int tile_rows;             // rows of a tile: BM, 2 BM for CTA pairs
+  bool vec_d, vec_aux, vec_bias;   // rows of the output / saved tensor and the bias start on 16-byte boundaries (set_vec)
   float alpha;
   float* ws;                 // splits>1: fp32 partial tiles, [tile][split][BM*BN]
   unsigned int* tile_ctr;    // splits>1: one arrival counter per tile (zero between launches)
@@ -223,7 +224,7 @@ __device__ __forceinline__ void epilogue_groups_bf16(const GemmParams& p, const 
   constexpr int NC = (BN < G ? BN : G) / 16;                      // 16-column chunks per group
   constexpr int RS = 32 / CPR;                                    // rows per copy instruction
   const int rr0 = lane / CPR, ch = lane % CPR;                    // copies: this lane's first row and its chunk of every row
-  const bool vec_d = p.ldd % 8 == 0, vec_a = p.ld_aux % 8 == 0;
+  const bool vec_d = p.vec_d, vec_a = p.vec_aux;
   uint4 ax[NV];
   auto load_aux = [&](int c) {
     const int col = n0 + c + ch * 8;
@@ -312,7 +313,7 @@ __device__ __forceinline__ void epilogue_groups_f32(const GemmParams& p, const f
                                                   int n0, int half, int lane, float* part) {
   constexpr int G = 32;
   constexpr int NC = (BN < G ? BN : G) / 16;
-  const bool vec_d = p.ldd % 4 == 0;
+  const bool vec_d = p.vec_d;
 #pragma unroll 1
   for (int c = half * G; c < BN && n0 + c < p.N; c += 2 * G) {
     auto chunk = [&](int k, const uint32_t* r) {
@@ -481,6 +482,14 @@ inline int sm_count() {
     if (n <= 0) n = 148;
   }
   return n;
+}
+
+// The base counts as well as the pitch: an output may be a few columns of a wider tensor.
+inline void set_vec(GemmParams& p) {
+  auto rows16 = [](const void* base, long long pitch) { return ((reinterpret_cast<uintptr_t>(base) | (uintptr_t)pitch) & 15) == 0; };
+  p.vec_d = rows16(p.D, (long long)p.ldd * (p.out_f32 ? 4 : 2));
+  p.vec_aux = rows16(p.aux, (long long)p.ld_aux * 2);
+  p.vec_bias = rows16(p.bias, 0);
 }
 
 // ---- choice of tile form and split

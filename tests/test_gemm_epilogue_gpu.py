@@ -47,3 +47,34 @@ def test_epilogue_edges(m, n, form, tiles):
     assert bool((err <= bound).all()), float((err - bound).max())
     if form == "pitch":
         assert bool((buf[:, n:] == 7.0).all())
+
+
+@pytest.mark.parametrize("n", [4, 8, 12, 15, 16, 40, 72])
+@pytest.mark.parametrize("shift", [1, 2, 3, 5])
+@pytest.mark.parametrize("k", [64, 4096])                   # one range of K, and split ranges with a second kernel
+@pytest.mark.parametrize("form", ["bf16", "f32", "accumulate", "residual"])
+def test_outputs_off_the_16_byte_grid(n, shift, k, form):
+    """Columns of a wider tensor whose pitch is a whole number of 16-byte words and whose base is not; residual and bias alike."""
+    from noeira_b200 import ops
+    g = torch.Generator(device="cuda").manual_seed(n * 100 + shift)
+    m = 37
+    a = torch.randn(m, k, device="cuda", generator=g).bfloat16()
+    b = torch.randn((n + 7) // 8 * 8, k, device="cuda", generator=g).bfloat16()[:n]
+    dt = torch.float32 if form in ("f32", "accumulate") else torch.bfloat16
+    buf = torch.full((m, 96), 7.0, device="cuda", dtype=dt)
+    out, kw = buf[:, shift:shift + n], {}
+    exact = a.double() @ b.double().t()
+    if form == "accumulate":
+        kw, exact = dict(accumulate=True), exact + 7.0
+    else:
+        bias = torch.randn(n + shift, device="cuda", generator=g)[shift:]
+        kw, exact = dict(bias=bias), exact + bias.double()
+        if form == "residual":
+            res = torch.randn(m, 96, device="cuda", generator=g).bfloat16()[:, shift:shift + n]
+            kw["residual"], exact = res, exact + res.double()
+    ops.gemm(a, b, out=out, n=n, **kw)
+    # one rounding to the result's type; k / 16 additions into an fp32 sum of order sqrt(k)
+    bound = (2.0 ** -8 if dt is torch.bfloat16 else 2.0 ** -22) * exact.abs() + (k / 16 + 4) * 2.0 ** -23 * 4 * k ** 0.5
+    err = (out.double() - exact).abs()
+    assert bool((err <= bound).all()), float((err - bound).max())
+    assert bool((buf[:, :shift] == 7.0).all()) and bool((buf[:, shift + n:] == 7.0).all())

@@ -478,7 +478,9 @@ mlp3_bwd_kernel(const __grid_constant__ MlpBwdGroup grp) {
     }
     bool ok = true;
     uint8_t* grow = sG + (r >> 3) * 1024 + (r & 7) * 128;
-    for (int layer = 0; layer < 2 && ok; ++layer) {
+    // A warp whose wait gave up does no further work but still takes part in the named barriers: the abort flag may be set
+    // between two warps' tests, and those that passed would wait there for ever.
+    for (int layer = 0; layer < 2; ++layer) {
       const __nv_bfloat16* hsrc = (layer == 0 ? p.h2 : p.h1) + (size_t)row * p.ld_h;
       const uint32_t acc = lane_addr + (uint32_t)(layer * 256 + half * 128);
       auto process = [&](const uint32_t (&cur)[32], const uint4 (&hv)[4], int s4) {
@@ -510,33 +512,35 @@ mlp3_bwd_kernel(const __grid_constant__ MlpBwdGroup grp) {
       uint4 ha[4], hb[4];
       load_h(ha, 0);          // ahead of the product they are multiplied with
       load_h(hb, 1);
-      if (!__all_sync(0xffffffffu, !*abort_flag && mbar_wait(&acc_full[layer], 0u, p.status, 350 + layer))) { ok = false; break; }
-      tc_fence_after();
-      tmem_ld_32x32b_x32_nowait(acc, ra);
-      tmem_ld_wait();
-      tmem_ld_32x32b_x32_nowait(acc + 32u, rb);
-      process(ra, ha, 0);
-      tmem_ld_wait();
-      tmem_ld_32x32b_x32_nowait(acc + 64u, ra);
-      load_h(ha, 2);
-      process(rb, hb, 1);
-      tmem_ld_wait();
-      tmem_ld_32x32b_x32_nowait(acc + 96u, rb);
-      load_h(hb, 3);
-      process(ra, ha, 2);
-      tmem_ld_wait();
-      process(rb, hb, 3);
-      if (layer == 0) {
-        tc_fence_before();
-        fence_proxy_async();
+      if (ok) ok = __all_sync(0xffffffffu, !*abort_flag && mbar_wait(&acc_full[layer], 0u, p.status, 350 + layer));
+      if (ok) {
+        tc_fence_after();
+        tmem_ld_32x32b_x32_nowait(acc, ra);
+        tmem_ld_wait();
+        tmem_ld_32x32b_x32_nowait(acc + 32u, rb);
+        process(ra, ha, 0);
+        tmem_ld_wait();
+        tmem_ld_32x32b_x32_nowait(acc + 64u, ra);
+        load_h(ha, 2);
+        process(rb, hb, 1);
+        tmem_ld_wait();
+        tmem_ld_32x32b_x32_nowait(acc + 96u, rb);
+        load_h(hb, 3);
+        process(ra, ha, 2);
+        tmem_ld_wait();
+        process(rb, hb, 3);
+        if (layer == 0) {
+          tc_fence_before();
+          fence_proxy_async();
+          __syncwarp();
+          if (lane == 0) mbar_arrive(g_ready);
+        }
         __syncwarp();
-        if (lane == 0) mbar_arrive(g_ready);
+        copy_tile_out(sG, layer == 0 ? p.g2 : p.g1, p.ld_g, row0, p.M, quarter, half, lane);
       }
-      __syncwarp();
-      copy_tile_out(sG, layer == 0 ? p.g2 : p.g1, p.ld_g, row0, p.M, quarter, half, lane);
       if (part) {
         asm volatile("bar.sync 1, 256;" ::: "memory");   // the whole tile is written
-        part[(layer == 0 ? HID : 0) + t] = tile_colsum(sG, t);       // [0] g1, [1] g2, [2] dy
+        if (ok) part[(layer == 0 ? HID : 0) + t] = tile_colsum(sG, t);       // [0] g1, [1] g2, [2] dy
         if (layer == 0) asm volatile("bar.sync 1, 256;" ::: "memory");   // sums read before layer 1 overwrites the tile
       }
     }

@@ -72,6 +72,7 @@ __device__ __forceinline__ void copy_tile_out(const uint8_t* tile, __nv_bfloat16
       if (row0 + rr < M) *reinterpret_cast<uint4*>(dst + (size_t)(row0 + rr) * ld + kb * 64 + ch * 8) = v;
     }
   }
+  __syncwarp();   // the next layer overwrites the rows that other lanes have read here
 }
 
 // blockIdx.y selects the network: the actor and the critic of an RL update run in ONE launch.

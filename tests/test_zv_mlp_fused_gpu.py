@@ -104,3 +104,23 @@ def test_fused_mlp_group_forward_backward_matches_layers(M):
             cos = torch.nn.functional.cosine_similarity(pa.grad.flatten(), pb.grad.flatten(), dim=0).item()
             rel = (pa.grad - pb.grad).abs().max().item() / max(pb.grad.abs().max().item(), 1e-6)
             assert cos > 0.999 and rel < 3e-2, (n, cos, rel)
+
+
+def test_fused_mlp_saves_repeat_bits():
+    """The saved activations and gradients leave a tile that the next layer overwrites: every run gives the same bits."""
+    from noeira_b200 import nn
+    from noeira_b200.ops import check_status
+    from noeira_b200.ops.mlp import Mlp3Pass, mlp3_backward_group, mlp3_forward_group
+    net = nn.Sequential(nn.Linear(17, 256, act="tanh", need_input_grad=False), nn.Linear(256, 256, act="tanh"),
+                        nn.Linear(256, 6, out_fp32=True)).to("cuda")
+    M = 148 * 128 + 77
+    x, dy = torch.randn(M, 24, device="cuda").bfloat16(), torch.randn(M, 8, device="cuda").bfloat16()
+    first = None
+    for _ in range(8):
+        p = Mlp3Pass(*net.mods, M, x.device)
+        mlp3_forward_group([p], [x])
+        mlp3_backward_group([p], [x], [dy])
+        got = [t.clone() for t in (p.out[:, :6], p.h1, p.h2, p.g1, p.g2)]
+        first = first or got
+        assert all(torch.equal(a, b) for a, b in zip(first, got))
+    check_status()

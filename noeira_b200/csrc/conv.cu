@@ -398,7 +398,7 @@ maxpool_fwd_kernel(const __nv_bfloat16* __restrict__ x, __nv_bfloat16* __restric
   for (int i = blockIdx.y * 256 + threadIdx.x; i < OW * CV; i += gridDim.y * 256) {
     const int ow = i / CV, c0 = (i - ow * CV) * VEC;
     float best[VEC];
-    I tap[VEC];
+    __align__(8) I tap[VEC];
 #pragma unroll
     for (int j = 0; j < VEC; ++j) { best[j] = -INFINITY; tap[j] = (I)-1; }
     const int K = KC ? KC : K_, h0 = oh * stride - pad, w0 = ow * stride - pad;
@@ -492,7 +492,7 @@ maxpool_bwd_kernel(const __nv_bfloat16* __restrict__ dy, const I* __restrict__ i
     auto tap_of = [&](int oh, int ow) { return (I)((h + pad - oh * stride) * K + (w + pad - ow * stride)); };
     for (int oh = oh_lo; oh <= oh_hi; ++oh)
       for (int ow = ow_lo; ow <= ow_hi; ++ow) {
-        I id[VEC];
+        __align__(8) I id[VEC];
         uint4 g = make_uint4(0, 0, 0, 0);
         load(oh, ow, id, g);
         add(id, g, tap_of(oh, ow));
@@ -568,7 +568,7 @@ image_normalize_kernel(const unsigned char* __restrict__ img, __nv_bfloat16* __r
   const long long px = ((long long)blockIdx.x * 256 + threadIdx.x) * PX;
   if (px >= HW) return;
   const unsigned char* p = img + (size_t)blockIdx.y * 3 * HW + px;
-  unsigned char v[3][PX];
+  __align__(4) unsigned char v[3][PX];
 #pragma unroll
   for (int c = 0; c < 3; ++c) {
     if (PX == 4) *reinterpret_cast<uint32_t*>(v[c]) = __ldg(reinterpret_cast<const uint32_t*>(p + (size_t)c * HW));

@@ -448,7 +448,7 @@ mlp3_bwd_kernel(const __grid_constant__ MlpBwdGroup grp) {
       uint4 c[2] = {zero4, zero4};
       if (grow_ < p.M) {
         const __nv_bfloat16* src = p.dy + (size_t)grow_ * p.ld_dy;
-        __nv_bfloat16 v[16];
+        __align__(16) __nv_bfloat16 v[16];
 #pragma unroll
         for (int j = 0; j < 16; ++j) v[j] = j < p.n3 ? src[j] : __float2bfloat16(0.f);
         c[0] = *reinterpret_cast<uint4*>(&v[0]);
@@ -461,7 +461,7 @@ mlp3_bwd_kernel(const __grid_constant__ MlpBwdGroup grp) {
     {
       const int n = t;
       const __nv_bfloat16* src = p.w3 + (size_t)n * p.ld_w3;
-      __nv_bfloat16 v[16];
+      __align__(16) __nv_bfloat16 v[16];
 #pragma unroll
       for (int j = 0; j < 16; ++j) v[j] = j < p.n3 ? src[j] : __float2bfloat16(0.f);
       uint8_t* dst = sW3 + (n >> 3) * 1024 + (n & 7) * 128;

@@ -603,6 +603,7 @@ int nb_im2col(const void* x, void* col, int B, int H, int W, int C, int KH, int 
 int nb_col2im(const void* dcol, void* dx, int B, int H, int W, int C, int KH, int KW, int stride, int pad, int OH, int OW,
               int ldc, void* stream) {
   if (C % 8 || ldc % 8) return NB_ERR_UNALIGNED;
+  if (B <= 0 || H <= 0 || W <= 0 || C <= 0) return NB_OK;   // an empty batch: a grid of no blocks is an error
   col2im_kernel<<<dim3((unsigned)(B * H), pool_blocks(W * (C / 8))), 256, 0, (cudaStream_t)stream>>>(
       (const __nv_bfloat16*)dcol, (__nv_bfloat16*)dx, H, W, C, KH, KW, stride, pad, OH, OW, ldc);
   NB_LAUNCH_CHECK();
@@ -660,6 +661,7 @@ int nb_bn_bwd(const void* dy, const void* x, const void* relu_out, const float* 
 int nb_maxpool_idx_bytes(int K) { return K * K < 255 ? 1 : 4; }
 int nb_maxpool_fwd(const void* x, void* y, void* idx, int B, int H, int W, int C, int K, int stride, int pad, int OH, int OW,
                    void* stream) {
+  if (B <= 0 || OH <= 0 || OW <= 0 || C <= 0) return NB_OK;
   cudaStream_t s = (cudaStream_t)stream;
   const bool vec = C % 8 == 0 && ((reinterpret_cast<uintptr_t>(x) | reinterpret_cast<uintptr_t>(y)) & 15) == 0 &&
                    (reinterpret_cast<uintptr_t>(idx) & 7) == 0;
@@ -681,6 +683,7 @@ int nb_maxpool_fwd(const void* x, void* y, void* idx, int B, int H, int W, int C
 }
 int nb_maxpool_bwd(const void* dy, const void* idx, void* dx, int B, int H, int W, int C, int K, int stride, int pad, int OH,
                    int OW, void* stream) {
+  if (B <= 0 || H <= 0 || W <= 0 || C <= 0) return NB_OK;
   cudaStream_t s = (cudaStream_t)stream;
   const bool vec = C % 8 == 0 && ((reinterpret_cast<uintptr_t>(dy) | reinterpret_cast<uintptr_t>(dx)) & 15) == 0 &&
                    (reinterpret_cast<uintptr_t>(idx) & 7) == 0;
@@ -721,7 +724,7 @@ int nb_upsample_nearest(const void* src, void* dst, int B, int H, int W, int C, 
 int nb_image_normalize(const unsigned char* img, void* out, int B, int H, int W, float m0, float m1, float m2, float s0,
                        float s1, float s2, void* stream) {
   const long long hw = (long long)H * W;
-  if (B <= 0 || hw <= 0) return NB_ERR_BAD_ARG;
+  if (B <= 0 || hw <= 0) return NB_OK;
   const bool by4 = hw % 4 == 0 && (reinterpret_cast<uintptr_t>(img) & 3) == 0;
   for (int b0 = 0; b0 < B; b0 += 65535) {          // grid.y limit
     const int n = B - b0 < 65535 ? B - b0 : 65535;

@@ -452,6 +452,7 @@ int nb_add_bf16(const void* a, const void* b, void* y, long long n, void* stream
 
 int nb_swiglu_fwd(const void* gu, int ld, void* h, int ldh, int M, int H, void* stream) {
   if (H % 2 || ld % 2 || ldh % 2) return NB_ERR_UNALIGNED;
+  if (M <= 0 || H <= 0) return NB_OK;
   if (H % 8 == 0 && ld % 8 == 0 && ldh % 8 == 0 && aligned16(gu, h)) {
     swiglu_fwd_vec_kernel<<<row_grid(M, H), 256, 0, (cudaStream_t)stream>>>((const __nv_bfloat16*)gu, ld, (__nv_bfloat16*)h, ldh, M, H);
     NB_LAUNCH_CHECK();
@@ -465,6 +466,7 @@ int nb_swiglu_fwd(const void* gu, int ld, void* h, int ldh, int M, int H, void* 
 
 int nb_swiglu_bwd(const void* gu, int ld, const void* dh, int ldh, void* dgu, int M, int H, void* stream) {
   if (H % 2 || ld % 2 || ldh % 2) return NB_ERR_UNALIGNED;
+  if (M <= 0 || H <= 0) return NB_OK;
   if (H % 8 == 0 && ld % 8 == 0 && ldh % 8 == 0 && aligned16(gu, dh, dgu)) {
     swiglu_bwd_vec_kernel<<<row_grid(M, H), 256, 0, (cudaStream_t)stream>>>((const __nv_bfloat16*)gu, ld, (const __nv_bfloat16*)dh, ldh,
                                                                            (__nv_bfloat16*)dgu, M, H);

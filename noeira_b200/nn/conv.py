@@ -43,12 +43,19 @@ def _aligned(t):
     return t if t.data_ptr() % 16 == 0 else t.clone()
 
 
+def _gather_fits(B, H, W, C, k, stride, pad):
+    """Sizes whose offsets the gathering kernel can hold in 32 bits: ``conv_fits`` of csrc/conv_index.h, which refuses the rest."""
+    OH, OW = (H + 2 * pad - k) // stride + 1, (W + 2 * pad - k) // stride + 1
+    return (B * H + 2 * pad) * (W + 2 * pad) * C <= (1 << 31) - 1 and B * OH * OW <= (1 << 31) - 1 - 256
+
+
 class Conv2D(Module):
     def __init__(self, ic, oc, k, stride=1, pad=0, bias=True, relu=False, need_input_grad=True):
         super().__init__()
         self.ic, self.oc, self.k, self.stride, self.pad, self.relu = ic, oc, k, stride, pad, relu
         self.icp = (ic + 7) // 8 * 8          # channels as stored (stem: 3 → 8, extra channels are zero)
         self.need_input_grad = need_input_grad
+        self._in = (1, 1, 1)                  # B, H, W of the last forward
         # False: patch matrix in memory (im2col) instead of the gathering convolution kernel
         self.implicit_gemm = os.environ.get("NOEIRA_B200_IMPLICIT_CONV", "1") != "0"
         self.weight = self.add_param("weight", (k * k * self.icp, oc), decay=True, init=Kaiming(), fan_in=ic * k * k,
@@ -66,8 +73,7 @@ class Conv2D(Module):
         """The gathering kernel takes every stride, padding and width; its offsets are 32-bit."""
         if not self.implicit_gemm or C % 8:
             return False
-        B, H, W = getattr(self, "_in", (1, 1, 1))
-        return (B * H + 2 * self.pad) * (W + 2 * self.pad) * C < 1 << 31 and B * (H + 2 * self.pad) * OW < (1 << 31) - 256
+        return _gather_fits(*self._in, C, self.k, self.stride, self.pad)
 
     def _implicit_wgrad_ok(self, OW):
         return self._implicit_ok(self.icp, OW)
@@ -196,8 +202,9 @@ class Conv2D(Module):
         dy (taps mirrored, channel roles swapped), without the k² times larger patch-gradient matrix and the pass over it."""
         if self.stride != 1 or self.k == 1 or self.oc % 64 or not self.implicit_gemm or self.pad > self.k - 1:
             return False
-        B, H, _ = getattr(self, "_in", (1, 1, 1))
-        return (B * H + 4 * self.k) * (W + 4 * self.k) * max(self.oc, self.icp) < 1 << 31
+        B, H, W = self._in
+        OH, OW = self.out_hw(H, W)                 # more than H by up to k − 1 per image
+        return _gather_fits(B, OH, OW, self.oc, self.k, 1, self.k - 1 - self.pad)
 
     def _implicit_dgrad(self, d2, B, H, W, OH, OW):
         dyc = _aligned(d2).view(B, OH, OW, self.oc)

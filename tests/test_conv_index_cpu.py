@@ -36,3 +36,26 @@ def test_gather_stays_inside_the_input(c, k, stride, pad, b, h, w, wgrad):
     full = np.full((rows, chunks), -1, np.int64)             # pixels past the last and taps past the last are zeros
     full[: want.shape[0], : want.shape[1]] = want
     assert np.array_equal(off, full)
+
+
+def test_host_guards_are_the_kernels():
+    """A layer chooses the gathering kernel exactly for the sizes that the kernel takes, in both directions."""
+    from noeira_b200 import nn
+    from noeira_b200.nn.conv import _gather_fits
+    fits = lambda *v: bool(host_lib().nbh_conv_fits(*(ctypes.c_int(i) for i in v)))
+    rng = np.random.default_rng(0)
+    both = set()
+    for _ in range(3000):
+        k, stride = int(rng.integers(1, 8)), int(rng.integers(1, 4))
+        pad, c, h, w = int(rng.integers(0, k)), 8 * int(rng.integers(1, 33)), int(rng.integers(k, 60)), int(rng.integers(k, 3000))
+        b = max(1, int(2 ** 31 / (h * w * c) * rng.uniform(0.4, 1.5)))
+        got = fits(b, h, w, c, k, k, stride, pad)
+        assert _gather_fits(b, h, w, c, k, stride, pad) == got
+        both.add(got)
+    assert both == {True, False}
+    # dy of a 'full' layer is larger than x: 20000 x 3 x 1002 x 64 elements for 20000 x 1 x 1000 x 64
+    conv = nn.Conv2D(64, 64, 3, 1, 2)
+    for b in (10000, 11159, 11165, 20000, 40000):
+        conv._in = (b, 1, 1000)
+        assert conv._implicit_dgrad_ok(1000) == fits(b, 3, 1002, 64, 3, 3, 1, 0)
+        assert conv._implicit_ok(64, 1002) == fits(b, 1, 1000, 64, 3, 3, 1, 2)

@@ -16,25 +16,12 @@ from .. import ops
 from .._native import check, cuda_lib, ptr, raw_stream, stream_ptr
 from ..ops.gemm import ACT, _workspace
 from ..ops.status import status_ptr
+from ..ops.streams import Scratch
 from .init import Constant, Kaiming, Zero
 from .layers import colsum_into
 from .module import Module
 
-_WS = {}
-_WS_KEPT = []
-
-
-def _scratch(device, n):
-    from ..ops.streams import ws_key
-    key = ws_key(device)
-    t = _WS.get(key)
-    if t is None or t.numel() < n:
-        # a captured graph may hold the smaller buffer's address: it stays alive, and doubling bounds what is kept
-        if t is not None:
-            _WS_KEPT.append(t)
-        t = torch.empty(max(n, 2 * t.numel() if t is not None else 1 << 20), dtype=torch.float32, device=device)
-        _WS[key] = t
-    return t
+_scratch = Scratch(1 << 20).get
 
 
 def _aligned(t):

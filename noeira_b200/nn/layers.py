@@ -13,6 +13,7 @@ import torch
 
 from .. import ops
 from .._native import check, cuda_lib, ptr, raw_stream, stream_ptr
+from ..ops.streams import Scratch
 from .init import Constant, Initializer, Kaiming, Zero
 from .module import Module
 
@@ -58,17 +59,7 @@ def _act_code(act):
     return ACT[act]
 
 
-_COLSUM_WS = {}
-
-
-def _colsum_workspace(device, need: int):
-    from ..ops.streams import ws_key
-    key = ws_key(device)
-    ws = _COLSUM_WS.get(key)
-    if ws is None or ws.numel() < need:
-        ws = torch.empty(max(need, 256 * 8192), dtype=torch.float32, device=device)
-        _COLSUM_WS[key] = ws
-    return ws
+_colsum_workspace = Scratch(256 * 8192).get
 
 
 def colsum_into(dy, out_f32, n, accumulate=True):

@@ -14,25 +14,12 @@ import torch
 from .. import ops
 from .._native import check, cuda_lib, ptr, raw_stream, stream_ptr
 from ..ops.attention import attention_reference, flash_attention_backward, flash_attention_forward
+from ..ops.streams import Scratch
 from .init import Constant, Normal, Zero
 from .layers import Linear
 from .module import Module
 
-_WS = {}
-_WS_KEPT = []
-
-
-def _scratch(device, n):
-    from ..ops.streams import ws_key
-    key = ws_key(device)
-    t = _WS.get(key)
-    if t is None or t.numel() < n:
-        # a captured graph may hold the smaller buffer's address: it stays alive, and doubling bounds what is kept
-        if t is not None:
-            _WS_KEPT.append(t)
-        t = torch.empty(max(n, 2 * t.numel() if t is not None else 1 << 20), dtype=torch.float32, device=device)
-        _WS[key] = t
-    return t
+_scratch = Scratch(1 << 20).get
 
 
 class _Norm(Module):

@@ -25,6 +25,27 @@ def ws_key(device) -> tuple:
     return (idx, slot())
 
 
+class Scratch:
+    """fp32 scratch memory per device and workspace slot, grown on demand and shared by the kernels of a module.  A captured
+    graph holds the address of the buffer it was captured with, so a buffer that became too small stays alive; doubling bounds
+    what is kept to the size of the newest."""
+
+    def __init__(self, floats: int):
+        self._floats = floats
+        self._now, self._kept = {}, []
+
+    def get(self, device, n: int) -> torch.Tensor:
+        key = ws_key(device)
+        t = self._now.get(key)
+        if t is None or t.numel() < n:
+            size = max(n, self._floats)
+            if t is not None:
+                self._kept.append(t)
+                size = max(n, 2 * t.numel())
+            t = self._now[key] = torch.empty(size, dtype=torch.float32, device=device)
+        return t
+
+
 class Branch:
     """``with Branch(stream, slot): …`` forks from the current stream on entry; ``join()`` makes the current
     stream wait for everything the branch launched.  Tensors produced inside must stay alive until the join."""

@@ -226,21 +226,27 @@ bn_bwd_finish_kernel(const float* __restrict__ p0, const float* __restrict__ p1,
   if (dbeta) dbeta[c] += s;
 }
 
-// y = relu?( (x - mean) * rstd * gamma + beta + residual? ); rstd null: from `var` (inference with running statistics)
+// y = relu?( (x - mean) * rstd * gamma + beta + residual? ).  run_mean given (inference): the statistics are the running ones, and
+// `mean` and `rstd` receive what was used, for a backward pass that may come after the running ones have changed.
 __global__ void __launch_bounds__(256)
-bn_apply_kernel(const __nv_bfloat16* __restrict__ x, const float* __restrict__ mean, const float* __restrict__ rstd,
-                const float* __restrict__ var, float eps, const float* __restrict__ gamma, const float* __restrict__ beta, const __nv_bfloat16* __restrict__ res,
-                __nv_bfloat16* __restrict__ y, long long M, int C, int relu) {
+bn_apply_kernel(const __nv_bfloat16* __restrict__ x, float* __restrict__ mean, float* __restrict__ rstd,
+                const float* __restrict__ run_mean, const float* __restrict__ run_var, float eps, const float* __restrict__ gamma,
+                const float* __restrict__ beta, const __nv_bfloat16* __restrict__ res, __nv_bfloat16* __restrict__ y, long long M, int C,
+                int relu) {
   const BnMap m = bn_map(C, blockIdx.x, gridDim.x);
   if (!m.active) return;
   float mu[8], rs[8], ga[8], be[8];
-  load8f(mean + m.ch, mu);
-  if (rstd) {
+  if (!run_mean) {
+    load8f(mean + m.ch, mu);
     load8f(rstd + m.ch, rs);
   } else {
-    load8f(var + m.ch, rs);
+    load8f(run_mean + m.ch, mu);
+    load8f(run_var + m.ch, rs);
 #pragma unroll
-    for (int k = 0; k < 8; ++k) rs[k] = rsqrtf(rs[k] + eps);
+    for (int k = 0; k < 8; ++k) {
+      rs[k] = rsqrtf(rs[k] + eps);
+      if (m.row == 0) { mean[m.ch + k] = mu[k]; rstd[m.ch + k] = rs[k]; }
+    }
   }
   load8f(gamma + m.ch, ga);
   load8f(beta + m.ch, be);
@@ -615,7 +621,7 @@ int nb_bn_split(long long M) {
   long long s = ceil_div_ll(M, BN_UNROLL);
   return (int)(s < 1 ? 1 : (s > 592 ? 592 : s));
 }
-// partials: 2 * nb_bn_split(M) * C floats.  rstd null (not in training): from run_var
+// partials: 2 * nb_bn_split(M) * C floats.  mean, rstd: the statistics of this call (inference: the running ones), for nb_bn_bwd
 int nb_bn_fwd(const void* x, const float* gamma, const float* beta, const void* residual, void* y, float* mean, float* rstd,
               float* run_mean, float* run_var, float* partials, long long M, int C, float eps, float momentum, int relu,
               int training, void* stream) {
@@ -631,8 +637,9 @@ int nb_bn_fwd(const void* x, const float* gamma, const float* beta, const void* 
                                                           run_var);
     NB_LAUNCH_CHECK();
   }
-  bn_apply_kernel<<<bn_grid(M, C, 1 << 20), 256, 0, s>>>((const __nv_bfloat16*)x, mean, rstd, run_var, eps, gamma, beta,
-                                                        (const __nv_bfloat16*)residual, (__nv_bfloat16*)y, M, C, relu);
+  bn_apply_kernel<<<bn_grid(M, C, 1 << 20), 256, 0, s>>>((const __nv_bfloat16*)x, mean, rstd, training ? nullptr : run_mean,
+                                                        run_var, eps, gamma, beta, (const __nv_bfloat16*)residual,
+                                                        (__nv_bfloat16*)y, M, C, relu);
   NB_LAUNCH_CHECK();
   return NB_OK;
 }

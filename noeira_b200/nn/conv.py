@@ -237,14 +237,14 @@ class BatchNorm2D(Module):
         xc = x if x.is_contiguous() else x.contiguous()
         self._x = xc
         y = torch.empty_like(xc)
-        self._mean = torch.empty(self.c, device=x.device) if self.training else self.running_mean.data
-        # inference: the kernel takes the running variance itself; a backward pass makes its rstd when it comes
-        self._rstdv = torch.empty(self.c, device=x.device) if self.training else None
+        # mean and rstd of this call (inference: the running ones as they are now), which vjp needs
+        self._stat = torch.empty(2 * self.c, dtype=torch.float32, device=x.device)
+        mean = self._stat.data_ptr()
         lib = cuda_lib()
         split = lib.nb_bn_split(ctypes.c_longlong(M))
         rc = residual.contiguous() if residual is not None else None
         check(lib.nb_bn_fwd(xc.data_ptr(), self.gamma.storage.data_ptr(), self.beta.storage.data_ptr(), None if rc is None else rc.data_ptr(),
-                            y.data_ptr(), self._mean.data_ptr(), self._rstdv.data_ptr() if self.training else None,
+                            y.data_ptr(), mean, mean + 4 * self.c,
                             self.running_mean.data.data_ptr(), self.running_var.data.data_ptr(),
                             _scratch(x.device, 2 * split * self.c).data_ptr(), M, self.c, self.eps, self.momentum, int(self.relu),
                             int(self.training), raw_stream()), "bn_fwd")
@@ -268,13 +268,12 @@ class BatchNorm2D(Module):
         d = dy if (dy.is_contiguous() and dy.dtype == torch.bfloat16) else dy.to(torch.bfloat16).contiguous()
         dx = torch.empty_like(d)
         dres = torch.empty_like(d) if self._has_res else None
-        if self._rstdv is None:
-            self._rstdv = torch.rsqrt(self.running_var.data + self.eps)
         lib = cuda_lib()
         split = lib.nb_bn_split(ctypes.c_longlong(M))
         ws = _scratch(dy.device, 2 * split * self.c + 2 * self.c)
         sums = ws[2 * split * self.c:]
-        check(lib.nb_bn_bwd(ptr(d), ptr(self._x), ptr(self._y if self.relu else None), ptr(self._mean), ptr(self._rstdv),
+        check(lib.nb_bn_bwd(ptr(d), ptr(self._x), ptr(self._y if self.relu else None), ptr(self._stat),
+                            ptr(self._stat[self.c:]),
                             ptr(self.gamma.storage), ptr(dx), ptr(dres), ptr(self.gamma.grad_storage), ptr(self.beta.grad_storage),
                             ptr(ws), ptr(sums), ctypes.c_longlong(M), ctypes.c_int(self.c), stream_ptr()), "bn_bwd")
         return (dx, dres) if self._has_res else dx

@@ -38,6 +38,37 @@ def test_batchnorm_edges(b, h, w, c, res):
         assert torch.equal(dres.double().reshape(-1, c), gm)
 
 
+@pytest.mark.parametrize("b,h,w,c", [(1, 1, 1, 8), (2, 7, 9, 64), (2, 5, 3, 2056), (3, 33, 31, 136)])
+@pytest.mark.parametrize("res", [False, True])
+def test_batchnorm_inference_backward_uses_the_forward_statistics(b, h, w, c, res):
+    """Running statistics that change between forward and vjp (weights loaded, an averaged copy swapped in) change neither."""
+    from noeira_b200 import nn
+    g = torch.Generator(device="cuda").manual_seed(c)
+    bn = nn.BatchNorm2D(c, relu=True).to("cuda").eval()
+    bn.gamma.set_(torch.rand(c) + 0.5)
+    bn.beta.set_(torch.randn(c))
+    bn.running_mean.data.copy_(torch.randn(c, device="cuda", generator=g))
+    bn.running_var.data.copy_(torch.rand(c, device="cuda", generator=g) + 0.25)
+    mean, rstd = bn.running_mean.data.double(), torch.rsqrt(bn.running_var.data.double() + bn.eps)
+    x = torch.randn(b, h, w, c, device="cuda", generator=g).bfloat16()
+    r = torch.randn(b, h, w, c, device="cuda", generator=g).bfloat16() if res else None
+    dy = torch.randn(b, h, w, c, device="cuda", generator=g).bfloat16()
+    y = bn.forward(x, residual=r)
+    bn.running_mean.data.fill_(100.0)
+    bn.running_var.data.fill_(100.0)
+    out = bn.vjp(dy)
+    dx = out[0] if res else out
+    M, ga = b * h * w, bn.gamma.data.double()
+    xh = (x.double().reshape(-1, c) - mean) * rstd
+    pre = xh * ga + bn.beta.data.double() + (r.double().reshape(-1, c) if res else 0)
+    assert torch.allclose(y.double().reshape(-1, c), pre.clamp_min(0), rtol=2 ** -8, atol=1e-4)
+    gm = dy.double().reshape(-1, c) * (y.reshape(-1, c) > 0)
+    tol = 1e-5 * M ** 0.5 + 1e-5                                      # fp32 sums of M terms of order one
+    assert torch.allclose(bn.gamma.grad.double(), (gm * xh).sum(0), rtol=1e-4, atol=10 * tol)
+    ref = ga * rstd * (gm - gm.mean(0) - xh * (gm * xh).mean(0))
+    assert torch.allclose(dx.double().reshape(-1, c), ref, rtol=2 ** -8, atol=2e-4 * max(1.0, float((ga * rstd).max())))
+
+
 @pytest.mark.parametrize("k,stride,pad", [(3, 2, 1), (3, 2, 0), (2, 2, 0), (5, 3, 2), (16, 4, 3), (1, 1, 0)])
 @pytest.mark.parametrize("b,h,w,c", [(2, 17, 19, 64), (1, 16, 30, 12), (3, 40, 21, 8)])
 def test_maxpool_edges(k, stride, pad, b, h, w, c):

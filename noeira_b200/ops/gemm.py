@@ -84,7 +84,7 @@ def gemm(a: torch.Tensor, b: torch.Tensor, *, a_mn: bool = False, b_mn: bool = F
         N = n
     if out is None:
         out = torch.empty(M, N, device=a.device, dtype=out_dtype)
-    ldd, sd = out.stride()
+    ldd, sd = out.stride(0), out.stride(-1)          # [M, N], and anything else whose rows are `ldd` apart
     assert sd == 1 and out.shape[0] == M
     out_f32 = out.dtype is torch.float32
     assert out_f32 or out.dtype is torch.bfloat16

@@ -78,3 +78,14 @@ def test_outputs_off_the_16_byte_grid(n, shift, k, form):
     err = (out.double() - exact).abs()
     assert bool((err <= bound).all()), float((err - bound).max())
     assert bool((buf[:, :shift] == 7.0).all()) and bool((buf[:, shift + n:] == 7.0).all())
+
+
+def test_output_of_another_rank():
+    """`out` may be [M] for one column or [M, 1, N]: rows are what its first stride says."""
+    from noeira_b200 import ops
+    a, b = torch.randn(40, 64, device="cuda").bfloat16(), torch.randn(8, 64, device="cuda").bfloat16()
+    ref = ops.gemm(a, b, out_dtype=torch.float32)
+    one, mid = torch.zeros(40, device="cuda"), torch.zeros(40, 1, 8, device="cuda")
+    ops.gemm(a, b[:1], out=one, n=1)
+    ops.gemm(a, b, out=mid)
+    assert torch.equal(mid[:, 0], ref) and torch.equal(one, ref[:, 0])

@@ -126,6 +126,11 @@ class TPBlock:
         self.replicated = [self.g1, self.g2]
 
 
+def workspace_floats(lib, rows: int, dim: int) -> int:
+    """Partial sums of the loss, and of the norm backward for the ``rows`` of a shard."""
+    return max(1 << 22, 2 * lib.nb_norm_split(ctypes.c_int(rows)) * dim)
+
+
 class WorldModel:
     """Trainer-facing model object: ``loss = model.train_step(latents, actions)``."""
 
@@ -174,7 +179,7 @@ class WorldModel:
         self.cb_qkv = mk((b0.hq + 2 * b0.hkv) * hd, d, "rs")
         self.loss_acc = torch.zeros(1, device=self.device)
         self.lib = cuda_lib()
-        self._ws = torch.empty(1 << 22, device=self.device)
+        self._ws = torch.empty(workspace_floats(self.lib, self.ms, d), device=self.device)
         # positional table for the shard rows (sinusoidal over the position inside the sequence)
         pos = (torch.arange(self.ms, device=self.device) + rank * self.ms) % self.S
         self.pos = nn.sincos_embed(pos.float() / 64.0, d, min_period=1.0, max_period=float(self.S)).contiguous()

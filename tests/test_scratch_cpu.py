@@ -22,3 +22,14 @@ def test_column_sums_and_norms_draw_from_growing_scratch():
     from noeira_b200.ops.streams import Scratch
     for get in (conv._scratch, transformer._scratch, layers._colsum_workspace):
         assert isinstance(get.__self__, Scratch)
+
+
+def test_world_model_workspace_holds_the_norm_partials():
+    import ctypes
+
+    from noeira_b200._native import cuda_lib
+    from noeira_b200.models.world_model import workspace_floats
+    lib = cuda_lib()
+    for rows in (1, 64, 1000, 16448, 1 << 20):
+        for dim in (64, 2048, 14336, 16384, 32768):
+            assert 2 * lib.nb_norm_split(ctypes.c_int(rows)) * dim <= workspace_floats(lib, rows, dim)

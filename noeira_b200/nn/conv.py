@@ -169,10 +169,11 @@ class Conv2D(Module):
 
     def _conv(self, x, w, y, oc, stride, pad, mirror, bias=None, act=None):
         B, H, W, C = x.shape
-        ws = _workspace(x)
+        ws = _workspace(x, optional=True)          # without one the kernel does not split the reduction
+        ws, n = (None, 0) if ws is None else (ws.data_ptr(), ws.numel())
         check(cuda_lib().nb_conv_gemm(x.data_ptr(), w.data_ptr(), y.data_ptr(), B, H, W, C, oc, self.k, self.k, stride, pad, int(mirror),
                                       w.stride(0), y.stride(0), None if bias is None else bias.data_ptr(), ACT[act],
-                                      status_ptr(x.get_device()), ws.data_ptr(), ws.numel(), raw_stream()), "conv_gemm")
+                                      status_ptr(x.get_device()), ws, n, raw_stream()), "conv_gemm")
 
     def _implicit_wgrad(self, d2, B, H, W):
         """dW += patches(x)ᵀ · dy with the patches gathered from the saved NHWC input."""

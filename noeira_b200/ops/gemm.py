@@ -33,9 +33,12 @@ def default_workspace(device) -> torch.Tensor:
     return w
 
 
-def _workspace(t: torch.Tensor) -> torch.Tensor:
+def _workspace(t: torch.Tensor, optional: bool = False):
+    """Workspace for kernels on ``t``'s device; ``optional``: None where one cannot be made (first use under capture)."""
     w = _WS.get((t.get_device(), slot()))
-    return w if w is not None else default_workspace(t.device)
+    if w is None and not (optional and torch.cuda.is_current_stream_capturing()):
+        w = default_workspace(t.device)
+    return w
 
 
 TWO_CTA_AUTO, TWO_CTA_OFF, TWO_CTA_FORCE = 0, 1, 2

@@ -53,3 +53,29 @@ def test_gathered_convolution_repeats_bits():
         y = c.forward(x)
         out.append((y.clone(), c.vjp(y).clone(), c.weight.grad.clone()))
     assert all(torch.equal(p, q) for p, q in zip(*out))
+
+
+def test_convolution_captured_before_any_eager_product():
+    """The forward needs no workspace: a graph may be captured before one exists on the device."""
+    from noeira_b200 import nn
+    from noeira_b200.ops import check_status, device_status
+    from noeira_b200.ops.gemm import _WS
+    device_status()
+    c = nn.Conv2D(512, 64, 3, 1, 1).to("cuda")               # long reduction, few tiles: splits when it has a workspace
+    x = torch.randn(1, 8, 16, 512, device="cuda").bfloat16()
+    c.weight.shadow
+    torch.cuda.synchronize()
+    kept = dict(_WS)
+    _WS.clear()
+    try:
+        g = torch.cuda.CUDAGraph()
+        with torch.cuda.graph(g):
+            y = c.forward(x)
+    finally:
+        _WS.update(kept)
+    g.replay()
+    torch.cuda.synchronize()
+    check_status()
+    z = c.forward(x)
+    # two orders of 4608 / 16 fp32 additions of partial sums below 4, one bf16 rounding each
+    assert torch.allclose(y.float(), z.float(), rtol=2 ** -7, atol=288 * 2 ** -23 * 8)

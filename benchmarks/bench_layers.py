@@ -1,5 +1,5 @@
 """Device-timed leaf kernels outside the GEMM / attention benchmarks: LayerNorm / RMSNorm forward + backward, Conv2D forward
-(implicit GEMM against the patch-matrix path), BatchNorm2D forward + backward, max-pool, the ray-traced camera.
+(gathering kernel against the patch-matrix path), BatchNorm2D forward + backward, max-pool, the ray-traced camera.
 
     python benchmarks/bench_layers.py [--iters 10] [--only norm|conv|bn|pool|ray]
 """
@@ -62,7 +62,6 @@ def main():
             a = nn.Conv2D(ic, oc, 3, 1, 1, bias=False).to("cuda")
             b = nn.Conv2D(ic, oc, 3, 1, 1, bias=False).to("cuda")
             b.implicit_gemm = False
-            a.force_implicit = True
             x = torch.randn(16, H, W, ic, device="cuda").bfloat16()
             ti = timeit(lambda: a.forward(x), args.iters, flush)
             tp = timeit(lambda: b.forward(x), args.iters, flush)

@@ -310,7 +310,6 @@ int conv_any(const ConvGeom& g, GemmParams& p, const void* Bmat, long long inner
   const bool have_ws = workspace && workspace_bytes > NB_GEMM_WS_COUNTERS * 4 + (1 << 20);
   const long long ws_bytes = have_ws ? workspace_bytes - NB_GEMM_WS_COUNTERS * 4 : 0;
   p.ws = have_ws ? (float*)((char*)workspace + NB_GEMM_WS_COUNTERS * 4) : nullptr;
-  p.tile_ctr = nullptr;
   const int num_kb = ceil_div(p.K, BK), sms = sm_count();
   int splits, sp, BN = 64;
   long long best = best_split(CONV_64, p.M, p.N, num_kb, ws_bytes, sms, &splits);

@@ -9,6 +9,6 @@
 // `dact` slot only: the aux tensor is ADDED to the result (residual connection fused into the epilogue)
 #define NB_AUX_ADD 16
 
-// Split-K workspace: the first NB_GEMM_WS_COUNTERS u32 are per-tile arrival counters (zero at rest),
+// Split-K workspace: the first NB_GEMM_WS_COUNTERS u32 are reserved (zero; no kernel reads them), and
 // fp32 partial tiles follow.
 #define NB_GEMM_WS_COUNTERS 1024

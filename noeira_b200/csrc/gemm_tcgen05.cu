@@ -680,7 +680,7 @@ static int gemm_any(int tf32, const void* A, const void* B, void* D, int M, int 
   const int elt = tf32 ? 4 : 2, bk = 128 / elt;   // elements per 128-byte row = k-block depth = MN-major chunk width
   if (accumulate && !out_f32) return NB_ERR_BAD_ARG;
   if (dact && !aux) return NB_ERR_BAD_ARG;
-  // workspace layout: [NB_GEMM_WS_COUNTERS u32 tile counters (zero at rest)] [fp32 partial tiles]
+  // workspace: fp32 partial tiles behind NB_GEMM_WS_COUNTERS words (gemm_api.h)
   const bool have_ws = workspace && workspace_bytes > NB_GEMM_WS_COUNTERS * 4 + (1 << 20);
   const long long ws_bytes = have_ws ? workspace_bytes - NB_GEMM_WS_COUNTERS * 4 : 0;
   const int num_kb = ceil_div(K, bk), sms = sm_count();
@@ -725,7 +725,6 @@ static int gemm_any(int tf32, const void* A, const void* B, void* D, int M, int 
   p.alpha = alpha;
   p.D = D; p.bias = bias; p.aux = (const __nv_bfloat16*)aux; p.status = status;
   p.ws = have_ws ? (float*)((char*)workspace + NB_GEMM_WS_COUNTERS * 4) : nullptr;
-  p.tile_ctr = have_ws ? (unsigned int*)workspace : nullptr;
   cudaStream_t s = (cudaStream_t)stream;
   if (two_cta) return launch_two_cta(tmA, tmB, p, splits, s);
   switch (BN) {

@@ -32,7 +32,6 @@ struct GemmParams {
   bool vec_d, vec_aux, vec_bias;   // rows of the output / saved tensor and the bias start on 16-byte boundaries (set_vec)
   float alpha;
   float* ws;                 // splits>1: fp32 partial tiles, [tile][split][BM*BN]
-  unsigned int* tile_ctr;    // splits>1: one arrival counter per tile (zero between launches)
   void* D;
   const float* bias;
   const __nv_bfloat16* aux;

@@ -26,7 +26,6 @@ constexpr int HID = 256;
 constexpr int ROWS = 128;
 constexpr int N3P = 16;
 constexpr int MLP_THREADS = 320;   // warp 0 TMA, warp 1 MMA, warps 2..9 epilogue (two warps per TMEM lane quarter)
-constexpr int EPI_THREADS = 256;
 
 struct MlpParams {
   int M, k0, n3;            // rows, input width (<= 64), real output width (<= 16)

@@ -63,20 +63,8 @@ class Conv2D(Module):
         return _gather_fits(*self._in, C, self.k, self.stride, self.pad)
 
     def _implicit_wgrad_ok(self, OW):
+        """The weight gradient gathers from the same input as the forward, within the same limits."""
         return self._implicit_ok(self.icp, OW)
-
-    def _patches(self):
-        """Patch matrix [B·OH·OW, KH·KW·C] of the saved input (backward of the implicit-GEMM forward)."""
-        x = self._xin
-        B, H, W, C = x.shape
-        OH, OW = self.out_hw(H, W)
-        K = self.k * self.k * C
-        if self._pointwise:
-            return x.reshape(B * OH * OW, C)
-        col = torch.empty(B * OH * OW, K, device=x.device, dtype=torch.bfloat16)
-        check(cuda_lib().nb_im2col(ptr(x), ptr(col), *(ctypes.c_int(v) for v in (B, H, W, C, self.k, self.k, self.stride,
-                                                                               self.pad, OH, OW, K)), stream_ptr()), "im2col")
-        return col
 
     def out_hw(self, H, W):
         return (H + 2 * self.pad - self.k) // self.stride + 1, (W + 2 * self.pad - self.k) // self.stride + 1
@@ -143,10 +131,10 @@ class Conv2D(Module):
             from .layers import act_backward
             d2 = act_backward(d2.contiguous(), self._y[:, : self.oc].contiguous() if self._y.shape[1] != self.oc else self._y, "relu")
         if not self.weight.frozen:
-            if self._col is None and not self._pointwise and self._implicit_wgrad_ok(OW):
+            if self._col is None and not self._pointwise:
                 self._implicit_wgrad(d2, B, H, W)
             else:
-                col = self._col if self._col is not None else self._patches()
+                col = self._col if self._col is not None else self._xin.reshape(-1, self.icp)
                 ops.gemm(col, d2, a_mn=True, b_mn=True, out=self.weight.grad_storage, accumulate=True, n=self.oc)
             if self.bias is not None:
                 colsum_into(d2, self.bias.grad_storage, self.oc)

@@ -450,7 +450,7 @@ maxpool_fwd_kernel(const __nv_bfloat16* __restrict__ x, __nv_bfloat16* __restric
         if (sizeof(I) == 1) *reinterpret_cast<uint2*>(idx + o) = *reinterpret_cast<const uint2*>(tap);
         else
 #pragma unroll
-          for (int q = 0; q < VEC; ++q) idx[o + q] = tap[q];
+          for (int q = 0; q < VEC; q += 4) *reinterpret_cast<int4*>(idx + o + q) = make_int4(tap[q], tap[q + 1], tap[q + 2], tap[q + 3]);
       } else {
         y[o] = __float2bfloat16(best[0]);
         idx[o] = tap[0];
@@ -461,7 +461,9 @@ maxpool_fwd_kernel(const __nv_bfloat16* __restrict__ x, __nv_bfloat16* __restric
 // dx = gather over the windows that contain the element (at most ceil(K/stride)^2 = 4 for 3x3 / 2): deterministic.
 // One thread owns VEC consecutive channels of one input pixel; the candidate output range is computed directly instead of
 // testing all K*K taps, and a window gives its gradient where its stored tap is the one that this pixel is for it.
-template <int VEC, typename I>
+// S1: the 3x3 / stride 1 window, whose nine windows are all loaded before the first is used (16 x 120 x 160 x 64: 74 us one by
+// one, 54 so; 4 x 56 x 56 x 64: 6.4, 4.6).
+template <int VEC, typename I, bool S1>
 __global__ void __launch_bounds__(256)
 maxpool_bwd_kernel(const __nv_bfloat16* __restrict__ dy, const I* __restrict__ idx, __nv_bfloat16* __restrict__ dx, int H, int W,
                    int C, int K, int stride, int pad, int OH, int OW) {
@@ -488,7 +490,10 @@ maxpool_bwd_kernel(const __nv_bfloat16* __restrict__ dy, const I* __restrict__ i
         if (sizeof(I) == 1) *reinterpret_cast<uint2*>(id) = __ldg(reinterpret_cast<const uint2*>(idx + o));
         else
 #pragma unroll
-          for (int q = 0; q < VEC; ++q) id[q] = idx[o + q];
+          for (int q = 0; q < VEC; q += 4) {
+            const int4 v = __ldg(reinterpret_cast<const int4*>(idx + o + q));
+            id[q] = (I)v.x; id[q + 1] = (I)v.y; id[q + 2] = (I)v.z; id[q + 3] = (I)v.w;
+          }
         g = __ldg(reinterpret_cast<const uint4*>(dy + o));
       } else {
         id[0] = idx[o];
@@ -496,6 +501,18 @@ maxpool_bwd_kernel(const __nv_bfloat16* __restrict__ dy, const I* __restrict__ i
       }
     };
     auto tap_of = [&](int oh, int ow) { return (I)((h + pad - oh * stride) * K + (w + pad - ow * stride)); };
+    if (S1) {
+      __align__(8) I id[9][VEC];
+      uint4 g[9];
+#pragma unroll
+      for (int t = 0; t < 9; ++t) {
+        const int oh = h + pad - t / 3, ow = w + pad - t % 3;              // this pixel is tap t of that window
+        if (oh >= 0 && oh < OH && ow >= 0 && ow < OW) load(oh, ow, id[t], g[t]);
+        else *reinterpret_cast<uint2*>(id[t]) = make_uint2(0xffffffffu, 0xffffffffu);     // no tap
+      }
+#pragma unroll
+      for (int t = 8; t >= 0; --t) add(id[t], g[t], (I)t);                 // windows in row order, as below
+    } else
     for (int oh = oh_lo; oh <= oh_hi; ++oh)
       for (int ow = ow_lo; ow <= ow_hi; ++ow) {
         __align__(8) I id[VEC];
@@ -664,18 +681,24 @@ int nb_bn_bwd(const void* dy, const void* x, const void* relu_out, const float* 
   return NB_OK;
 }
 
-// idx: one byte per output element when nb_maxpool_idx_bytes(K) == 1, else four
-int nb_maxpool_idx_bytes(int K) { return K * K < 255 ? 1 : 4; }
+// idx: one byte per output element when nb_maxpool_idx_bytes(K, stride) == 1, else four.  A pixel in more than nine windows takes
+// four: taking bytes out of words is then what the backward spends its time on (16 x 16 / 4 over 16 x 120 x 160 x 64: 139 us with bytes, 86
+// with words).
+int nb_maxpool_idx_bytes(int K, int stride) { return K * K < 255 && ceil_div(K, stride) <= 3 ? 1 : 4; }
 int nb_maxpool_fwd(const void* x, void* y, void* idx, int B, int H, int W, int C, int K, int stride, int pad, int OH, int OW,
                    void* stream) {
   if (B <= 0 || OH <= 0 || OW <= 0 || C <= 0) return NB_OK;
   cudaStream_t s = (cudaStream_t)stream;
-  const bool vec = C % 8 == 0 && ((reinterpret_cast<uintptr_t>(x) | reinterpret_cast<uintptr_t>(y)) & 15) == 0 &&
-                   (reinterpret_cast<uintptr_t>(idx) & 7) == 0;
+  // A large window is walked tap by tap, which needs threads to hide its latency: with few outputs, or few per row of blocks, a thread
+  // takes one channel instead of eight (us, eight / one: 8 x 8 / 8 over 16 x 56 x 56 x 64 18.5 / 6.2, 5 x 5 / 3 over 256 x 20 x 20 x 32
+  // 13.3 / 11.5; the other side, 5 x 5 / 3 over 16 x 56 x 56 x 64: 9.0 / 11.7).
+  const bool few = K >= 4 && ((long long)B * OH * OW * C < 148LL * 288 * 8 || OW * (C / 8) < 64);
+  const bool vec = !few && C % 8 == 0 && ((reinterpret_cast<uintptr_t>(x) | reinterpret_cast<uintptr_t>(y)) & 15) == 0 &&
+                   (reinterpret_cast<uintptr_t>(idx) & 15) == 0;
 #define NB_POOL(V, I, KC)                                                                                                   \
   maxpool_fwd_kernel<V, I, KC><<<dim3((unsigned)(B * OH), pool_blocks(OW * (C / V))), 256, 0, s>>>(                         \
       (const __nv_bfloat16*)x, (__nv_bfloat16*)y, (I*)idx, H, W, C, K, stride, pad, OH, OW)
-  const bool byte = nb_maxpool_idx_bytes(K) == 1;
+  const bool byte = nb_maxpool_idx_bytes(K, stride) == 1;
   if (vec) {
     if (K == 3) NB_POOL(8, unsigned char, 3);
     else if (byte) NB_POOL(8, unsigned char, 0);
@@ -693,21 +716,22 @@ int nb_maxpool_bwd(const void* dy, const void* idx, void* dx, int B, int H, int 
   if (B <= 0 || H <= 0 || W <= 0 || C <= 0) return NB_OK;
   cudaStream_t s = (cudaStream_t)stream;
   const bool vec = C % 8 == 0 && ((reinterpret_cast<uintptr_t>(dy) | reinterpret_cast<uintptr_t>(dx)) & 15) == 0 &&
-                   (reinterpret_cast<uintptr_t>(idx) & 7) == 0;
-#define NB_POOL(V, I)                                                                                                       \
-  maxpool_bwd_kernel<V, I><<<dim3((unsigned)(B * H), pool_blocks(W * (C / V))), 256, 0, s>>>(                               \
+                   (reinterpret_cast<uintptr_t>(idx) & 15) == 0;
+#define NB_POOL(V, I, S1)                                                                                                   \
+  maxpool_bwd_kernel<V, I, S1><<<dim3((unsigned)(B * H), pool_blocks(W * (C / V))), 256, 0, s>>>(                           \
       (const __nv_bfloat16*)dy, (const I*)idx, (__nv_bfloat16*)dx, H, W, C, K, stride, pad, OH, OW)
-  const bool byte = nb_maxpool_idx_bytes(K) == 1;
+  const bool byte = nb_maxpool_idx_bytes(K, stride) == 1;
   if (vec && K == 3 && stride == 2) {
     const int a0 = pad / 2, na = (H - 1 + pad) / 2 - a0 + 1, nw = (W - 1 + pad) / 2 - a0 + 1;   // pixel pairs per direction
     maxpool_bwd_3s2_kernel<<<dim3((unsigned)(B * na), pool_blocks(nw * (C / 8))), 256, 0, s>>>(
         (const __nv_bfloat16*)dy, (const unsigned char*)idx, (__nv_bfloat16*)dx, H, W, C, pad, OH, OW, a0, na, nw);
   } else if (vec) {
-    if (byte) NB_POOL(8, unsigned char);
-    else NB_POOL(8, int);
+    if (K == 3 && stride == 1) NB_POOL(8, unsigned char, true);
+    else if (byte) NB_POOL(8, unsigned char, false);
+    else NB_POOL(8, int, false);
   } else {
-    if (byte) NB_POOL(1, unsigned char);
-    else NB_POOL(1, int);
+    if (byte) NB_POOL(1, unsigned char, false);
+    else NB_POOL(1, int, false);
   }
 #undef NB_POOL
   NB_LAUNCH_CHECK();

@@ -283,8 +283,8 @@ class MaxPool2D(Module):
             return y.permute(0, 2, 3, 1)
         xc = x if x.is_contiguous() else x.contiguous()
         y = torch.empty(B, OH, OW, C, device=x.device, dtype=torch.bfloat16)
-        # which tap of its window was the maximum: a byte for all but very large windows
-        one = cuda_lib().nb_maxpool_idx_bytes(ctypes.c_int(self.k)) == 1
+        # which tap of its window was the maximum: a byte for all but large windows
+        one = cuda_lib().nb_maxpool_idx_bytes(ctypes.c_int(self.k), ctypes.c_int(self.stride)) == 1
         self._idx = torch.empty(B, OH, OW, C, device=x.device, dtype=torch.uint8 if one else torch.int32)
         check(cuda_lib().nb_maxpool_fwd(ptr(xc), ptr(y), ptr(self._idx), *(ctypes.c_int(v) for v in (B, H, W, C, self.k, self.stride,
                                                                                                  self.pad, OH, OW)), stream_ptr()), "maxpool_fwd")

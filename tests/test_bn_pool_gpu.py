@@ -5,7 +5,8 @@ import torch
 pytestmark = pytest.mark.gpu
 
 
-@pytest.mark.parametrize("b,h,w,c", [(1, 1, 2, 8), (1, 3, 5, 24), (2, 7, 9, 64), (3, 33, 31, 136), (2, 5, 3, 2056), (4, 61, 47, 512)])
+@pytest.mark.parametrize("b,h,w,c", [(1, 1, 2, 8), (1, 3, 5, 24), (2, 7, 9, 64), (3, 33, 31, 136), (2, 5, 3, 2056), (4, 61, 47, 512), (1, 33, 31, 8), (2, 3, 3, 2048),
+                                     (1, 8, 8, 256)])
 @pytest.mark.parametrize("res", [False, True])
 def test_batchnorm_edges(b, h, w, c, res):
     from noeira_b200 import nn
@@ -69,8 +70,8 @@ def test_batchnorm_inference_backward_uses_the_forward_statistics(b, h, w, c, re
     assert torch.allclose(dx.double().reshape(-1, c), ref, rtol=2 ** -8, atol=2e-4 * max(1.0, float((ga * rstd).max())))
 
 
-@pytest.mark.parametrize("k,stride,pad", [(3, 2, 1), (3, 2, 0), (2, 2, 0), (5, 3, 2), (16, 4, 3), (1, 1, 0)])
-@pytest.mark.parametrize("b,h,w,c", [(2, 17, 19, 64), (1, 16, 30, 12), (3, 40, 21, 8)])
+@pytest.mark.parametrize("k,stride,pad", [(3, 2, 1), (3, 2, 0), (2, 2, 0), (5, 3, 2), (16, 4, 3), (1, 1, 0), (3, 1, 1), (3, 1, 0), (4, 1, 2), (8, 8, 0)])
+@pytest.mark.parametrize("b,h,w,c", [(2, 17, 19, 64), (1, 16, 30, 12), (3, 40, 21, 8), (200, 20, 20, 32), (7, 90, 16, 64)])
 def test_maxpool_edges(k, stride, pad, b, h, w, c):
     from noeira_b200 import nn
     g = torch.Generator(device="cuda").manual_seed(k * 100 + c)

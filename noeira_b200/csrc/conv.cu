@@ -180,20 +180,20 @@ bn_reduce_kernel(const __nv_bfloat16* __restrict__ a, const __nv_bfloat16* __res
 constexpr int BN_FIN_WARPS = 32;
 __device__ __forceinline__ bool bn_finish_sums(const float* p0, const float* p1, int split, int C, int& c, float& s, float& ss) {
   __shared__ float q0[BN_FIN_WARPS][33], q1[BN_FIN_WARPS][33];
-  const int l = threadIdx.x & 31, w = threadIdx.x >> 5;
+  const int l = threadIdx.x & 31, w = threadIdx.x >> 5, warps = blockDim.x >> 5;
   c = blockIdx.x * 32 + l;
   float t0 = 0.f, t1 = 0.f;
   if (c < C) {
 #pragma unroll 8
-    for (int k = w; k < split; k += BN_FIN_WARPS) { t0 += p0[(size_t)k * C + c]; t1 += p1[(size_t)k * C + c]; }
+    for (int k = w; k < split; k += warps) { t0 += p0[(size_t)k * C + c]; t1 += p1[(size_t)k * C + c]; }
   }
   q0[w][l] = t0;
   q1[w][l] = t1;
   __syncthreads();
   s = ss = 0.f;
   if (w == 0) {
-#pragma unroll
-    for (int k = 0; k < BN_FIN_WARPS; ++k) { s += q0[k][l]; ss += q1[k][l]; }
+#pragma unroll 8
+    for (int k = 0; k < warps; ++k) { s += q0[k][l]; ss += q1[k][l]; }
   }
   return w == 0 && c < C;
 }
@@ -328,12 +328,17 @@ bn_bwd_dx_kernel(const __nv_bfloat16* __restrict__ dy, const __nv_bfloat16* __re
   }
 }
 
-// grid of the row-walking kernels: up to `blocks` blocks, each thread with at least one round of BN_UNROLL rows
+// grid of the row-walking kernels: up to `blocks` blocks, each thread with a round of BN_UNROLL rows, or with fewer while that
+// leaves less than BN_FIN_WARPS blocks (the finish takes a partial per warp).  Forward + backward, us, four rows / fewer: 1024 x 8
+// 18.0 / 16.0, 64 x 256 17.3 / 15.4; more blocks than that cost more in the finish (1024 x 512 with 149 blocks 19.5 / 23.7)
 inline dim3 bn_grid(long long M, int C, int blocks) {
   const int cv = C / 8, lanes = cv < 256 ? cv : 256, per = 256 / lanes;
-  const long long b = ceil_div_ll(M, (long long)per * BN_UNROLL);
+  const long long one = ceil_div_ll(M, per), four = ceil_div_ll(M, (long long)per * BN_UNROLL);
+  const long long b = four >= BN_FIN_WARPS ? four : (one < BN_FIN_WARPS ? one : BN_FIN_WARPS);
   return dim3((unsigned)(b < 1 ? 1 : (b > blocks ? blocks : b)), (unsigned)ceil_div(cv, lanes));
 }
+// a warp per partial
+inline int bn_fin_threads(unsigned split) { return 32 * (int)(split < (unsigned)BN_FIN_WARPS ? split : (unsigned)BN_FIN_WARPS); }
 
 // Average pooling with window K, stride = K (non-overlapping) on NHWC: forward averages, backward spreads dy / K².
 // `back != 0`: `src` is dy [B, OH, OW, C] and `dst` is dx [B, H, W, C] (pixels outside the pooled area get zero).
@@ -633,11 +638,8 @@ int nb_col2im(const void* dcol, void* dx, int B, int H, int W, int C, int KH, in
   return NB_OK;
 }
 
-// blocks of the statistics pass = number of partials: four blocks per SM
-int nb_bn_split(long long M) {
-  long long s = ceil_div_ll(M, BN_UNROLL);
-  return (int)(s < 1 ? 1 : (s > 592 ? 592 : s));
-}
+// most blocks of the statistics pass = most partials: four blocks per SM
+int nb_bn_split(long long M) { return (int)(M < 1 ? 1 : (M > 592 ? 592 : M)); }
 // partials: 2 * nb_bn_split(M) * C floats.  mean, rstd: the statistics of this call (inference: the running ones), for nb_bn_bwd
 int nb_bn_fwd(const void* x, const float* gamma, const float* beta, const void* residual, void* y, float* mean, float* rstd,
               float* run_mean, float* run_var, float* partials, long long M, int C, float eps, float momentum, int relu,
@@ -650,7 +652,7 @@ int nb_bn_fwd(const void* x, const float* gamma, const float* beta, const void* 
     float* p1 = partials + (size_t)g.x * C;
     bn_reduce_kernel<false><<<g, 256, 0, s>>>((const __nv_bfloat16*)x, nullptr, nullptr, nullptr, nullptr, p0, p1, M, C);
     NB_LAUNCH_CHECK();
-    bn_stats_finish_kernel<<<ceil_div(C, 32), 32 * BN_FIN_WARPS, 0, s>>>(p0, p1, (int)g.x, M, C, eps, momentum, mean, rstd, run_mean,
+    bn_stats_finish_kernel<<<ceil_div(C, 32), bn_fin_threads(g.x), 0, s>>>(p0, p1, (int)g.x, M, C, eps, momentum, mean, rstd, run_mean,
                                                           run_var);
     NB_LAUNCH_CHECK();
   }
@@ -672,7 +674,7 @@ int nb_bn_bwd(const void* dy, const void* x, const void* relu_out, const float* 
   bn_reduce_kernel<true><<<g, 256, 0, s>>>((const __nv_bfloat16*)dy, (const __nv_bfloat16*)x, mean, rstd,
                                           (const __nv_bfloat16*)relu_out, p0, p1, M, C);
   NB_LAUNCH_CHECK();
-  bn_bwd_finish_kernel<<<ceil_div(C, 32), 32 * BN_FIN_WARPS, 0, s>>>(p0, p1, (int)g.x, C, sums, sums + C, dgamma, dbeta);
+  bn_bwd_finish_kernel<<<ceil_div(C, 32), bn_fin_threads(g.x), 0, s>>>(p0, p1, (int)g.x, C, sums, sums + C, dgamma, dbeta);
   NB_LAUNCH_CHECK();
   bn_bwd_dx_kernel<<<bn_grid(M, C, 1 << 20), 256, 0, s>>>((const __nv_bfloat16*)dy, (const __nv_bfloat16*)x,
                                                          (const __nv_bfloat16*)relu_out, mean, rstd, gamma, sums, sums + C,

@@ -318,6 +318,11 @@ int noalloc_scratch(float** out) {
 inline bool aligned16(const void* a, const void* b = nullptr, const void* c = nullptr) {
   return ((reinterpret_cast<uintptr_t>(a) | reinterpret_cast<uintptr_t>(b) | reinterpret_cast<uintptr_t>(c)) & 15) == 0;
 }
+// Where rows of vectors beat the pair kernels (us, pairs / vectors).  Short tensors: the pair kernels' threads do not all have work yet,
+// and a thread with eight exponentials and divisions in a row is the longer chain (forward 128 x 2048 2.9 / 3.3, 256 x 2048 3.4 / 3.2).
+// Narrow rows: a block per row leaves most of its 256 threads idle (131072 x 64 19 / 81, backward 32768 x 400 34 / 43; x 512 43.3 / 43.7, forward
+// 40.6 / 33.9).
+inline bool wide_enough(long long rows, int H) { return H >= 512 && rows * H >= 1LL << 19; }
 // rows x 8-column vectors: enough blocks for four per SM and one round of two rows each, at most 65535 rows of blocks
 inline dim3 row_grid(int M, int H) {
   const int bx = ceil_div(H / 8, 256);
@@ -453,7 +458,7 @@ int nb_add_bf16(const void* a, const void* b, void* y, long long n, void* stream
 int nb_swiglu_fwd(const void* gu, int ld, void* h, int ldh, int M, int H, void* stream) {
   if (H % 2 || ld % 2 || ldh % 2) return NB_ERR_UNALIGNED;
   if (M <= 0 || H <= 0) return NB_OK;
-  if (H % 8 == 0 && ld % 8 == 0 && ldh % 8 == 0 && aligned16(gu, h)) {
+  if (wide_enough(M, H) && H % 8 == 0 && ld % 8 == 0 && ldh % 8 == 0 && aligned16(gu, h)) {
     swiglu_fwd_vec_kernel<<<row_grid(M, H), 256, 0, (cudaStream_t)stream>>>((const __nv_bfloat16*)gu, ld, (__nv_bfloat16*)h, ldh, M, H);
     NB_LAUNCH_CHECK();
     return NB_OK;
@@ -467,7 +472,7 @@ int nb_swiglu_fwd(const void* gu, int ld, void* h, int ldh, int M, int H, void* 
 int nb_swiglu_bwd(const void* gu, int ld, const void* dh, int ldh, void* dgu, int M, int H, void* stream) {
   if (H % 2 || ld % 2 || ldh % 2) return NB_ERR_UNALIGNED;
   if (M <= 0 || H <= 0) return NB_OK;
-  if (H % 8 == 0 && ld % 8 == 0 && ldh % 8 == 0 && aligned16(gu, dh, dgu)) {
+  if (wide_enough(M, H) && H % 8 == 0 && ld % 8 == 0 && ldh % 8 == 0 && aligned16(gu, dh, dgu)) {
     swiglu_bwd_vec_kernel<<<row_grid(M, H), 256, 0, (cudaStream_t)stream>>>((const __nv_bfloat16*)gu, ld, (const __nv_bfloat16*)dh, ldh,
                                                                            (__nv_bfloat16*)dgu, M, H);
     NB_LAUNCH_CHECK();

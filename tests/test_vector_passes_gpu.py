@@ -38,7 +38,8 @@ def test_norm_backward(m, d, rms):
         assert torch.allclose(n.beta.grad.double(), be.grad, rtol=1e-5, atol=tol)
 
 
-@pytest.mark.parametrize("m,h,extra", [(1, 8, 0), (3, 10, 0), (67, 2056, 0), (5, 24, 8), (5, 24, 2), (300, 2048, 0)])
+@pytest.mark.parametrize("m,h,extra", [(1, 8, 0), (3, 10, 0), (67, 2056, 0), (5, 24, 8), (5, 24, 2), (300, 2048, 0),
+                                       (70001, 8, 0), (8191, 72, 0), (2700, 200, 8), (1100, 512, 8), (257, 2056, 0), (25, 22536, 0)])
 def test_swiglu(m, h, extra):
     from noeira_b200 import nn
     g = _g(m + h)
@@ -62,7 +63,7 @@ def test_swiglu(m, h, extra):
         assert torch.allclose(dgu.double(), gd.grad, rtol=2 ** -8 + 1e-5, atol=1e-6)
 
 
-@pytest.mark.parametrize("n", [1, 7, 8, 4097, 100000])
+@pytest.mark.parametrize("n", [1, 7, 8, 4097, 100000, (1 << 18) - 1, (1 << 18) + 5])
 @pytest.mark.parametrize("off", [0, 1])
 @pytest.mark.parametrize("act", ["relu", "gelu", "silu"])
 def test_activation(n, off, act):
@@ -79,7 +80,8 @@ def test_activation(n, off, act):
     assert torch.allclose(dx.double(), xd.grad, rtol=2 ** -8 + 1e-5, atol=2e-6)
 
 
-@pytest.mark.parametrize("b,s,h,d", [(1, 1, 1, 16), (2, 33, 5, 64), (3, 7, 15, 128), (2, 9, 3, 8), (1, 300, 6, 48)])
+@pytest.mark.parametrize("b,s,h,d", [(1, 1, 1, 16), (2, 33, 5, 64), (3, 7, 15, 128), (2, 9, 3, 8), (1, 300, 6, 48), (2, 401, 7, 64), (3, 300, 9, 48),
+                                     (17, 300, 1, 64)])
 @pytest.mark.parametrize("packed", [False, True])
 def test_rope(b, s, h, d, packed):
     from noeira_b200.nn import rope_

@@ -440,7 +440,8 @@ int nb_act_fwd(const void* x, void* y, long long n, int act, void* stream) {
 }
 
 int nb_act_bwd(const void* dy, const void* saved, void* dx, long long n, int act, void* stream) {
-  const long long n8 = aligned16(dy, saved, dx) ? n / 8 : 0;
+  // short tensors: one element per thread is the shorter chain (SiLU, 65536 elements 2.2 us against 3.1 in vectors, 300000: 3.05 / 3.14)
+  const long long n8 = n >= (1 << 18) && aligned16(dy, saved, dx) ? n / 8 : 0;
   act_bwd_kernel<<<grid1d(n8 ? n8 : n), 256, 0, (cudaStream_t)stream>>>((const __nv_bfloat16*)dy, (const __nv_bfloat16*)saved,
                                                                        (__nv_bfloat16*)dx, n8, n, act);
   NB_LAUNCH_CHECK();

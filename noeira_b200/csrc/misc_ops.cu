@@ -292,7 +292,9 @@ extern "C" {
 int nb_rope(void* x, int B, int S, int H, int D, long long sb, long long ss, long long sh, float theta, int pos0,
             int backward, void* stream) {
   if (D % 2) return NB_ERR_BAD_ARG;
-  if (D % 16 == 0 && sb % 8 == 0 && ss % 8 == 0 && sh % 8 == 0 && (reinterpret_cast<uintptr_t>(x) & 15) == 0) {
+  // fewer than 1024 pairs per SM: a thread's eight sines in a row take longer than one each in the kernel above (256 tokens x 15 x 64:
+  // 3.0 us against 3.5; 512 tokens: 4.0 / 3.5)
+  if ((long long)B * S * H * (D / 2) >= 148 * 1024 && D % 16 == 0 && sb % 8 == 0 && ss % 8 == 0 && sh % 8 == 0 && (reinterpret_cast<uintptr_t>(x) & 15) == 0) {
     const long long n = (long long)B * S * ceil_div(H, ROPE_HEADS) * (D / 16);
     const long long blocks = (n + 127) / 128;
     rope_vec_kernel<<<(int)(blocks < 1 ? 1 : (blocks > 148 * 16 ? 148 * 16 : blocks)), 128, 0, (cudaStream_t)stream>>>(

@@ -393,7 +393,10 @@ int nb_norm_bwd(const void* x, int ldx, const void* dy, int lddy, const float* g
   if (D % 8 || ldx % 8 || lddy % 8 || lddx % 8) return NB_ERR_UNALIGNED;
   cudaStream_t s = (cudaStream_t)stream;
   dim3 grid(ceil_div(M, 8));
-  if (D <= MAXV * 256 && (dx || dgamma)) {
+  // a few LayerNorm rows wider than 512 take the separate kernels: adding up the 16 warps' sums, most of them empty, takes longer
+  // than the extra launch (1 x 1024: 8.7 us fused, 7.3 so; 16 x 1024: 9.8, 9.8)
+  const bool few = !rms && D > 512 && M <= 8;
+  if (D <= MAXV * 256 && !few && (dx || dgamma)) {
     const int split = nb_norm_split(M), need = ceil_div(D, 256);
     float* pg = dgamma ? partials : nullptr;
     float* pb = (rms || !dbeta || !dgamma) ? nullptr : partials + (size_t)split * D;
@@ -420,7 +423,7 @@ int nb_norm_bwd(const void* x, int ldx, const void* dy, int lddy, const float* g
     }
     return NB_OK;
   }
-  // wider rows: one kernel for dx, one for the parameter gradients
+  // wider or few rows: one kernel for dx, one for the parameter gradients
   if (dx) {
     if (rms)
       norm_bwd_dx_kernel<true><<<grid, 256, 0, s>>>((const __nv_bfloat16*)x, ldx, (const __nv_bfloat16*)dy, lddy, gamma,
@@ -432,7 +435,9 @@ int nb_norm_bwd(const void* x, int ldx, const void* dy, int lddy, const float* g
     NB_LAUNCH_CHECK();
   }
   if (dgamma) {
-    const int split = nb_norm_split(M);
+    // 64 rows per partial, and eight partials before that: with a partial per 8 rows the finish reads too many of these wide rows
+    // (LayerNorm, 4096 columns: 64 rows 21.5 us with one partial, 20.0 with eight; 1000 rows 24.8 with 15, 32.2 with 125)
+    const int split = M >= 512 ? (M / 64 < 128 ? M / 64 : 128) : (M >= 64 ? 8 : nb_norm_split(M));
     const int rows = ceil_div(M, split);
     float* pg = partials;
     float* pb = (rms || !dbeta) ? nullptr : partials + (size_t)split * D;

@@ -37,6 +37,8 @@ def _gather_fits(B, H, W, C, k, stride, pad):
 
 
 class Conv2D(Module):
+    """NHWC convolution.  The input is kept for ``vjp`` by reference, as the dense layers keep theirs: it must not change in between."""
+
     def __init__(self, ic, oc, k, stride=1, pad=0, bias=True, relu=False, need_input_grad=True):
         super().__init__()
         self.ic, self.oc, self.k, self.stride, self.pad, self.relu = ic, oc, k, stride, pad, relu

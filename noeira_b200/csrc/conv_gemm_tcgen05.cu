@@ -244,7 +244,7 @@ conv_gemm_kernel(const __grid_constant__ CUtensorMap tmB, const GemmParams p, co
       const int row_in_tile = quarter * 32, row0 = mb * BM + row_in_tile, n0 = nb_ * BN;
       constexpr int G = MODE == EPI_F32 ? 32 : epi_group<BN>();
       const float4 bias0 = load_bias<BN, G>(p, n0, 0, lane), bias1 = load_bias<BN, G>(p, n0, 1, lane);
-      if (!wait_or_abort(&tfull_bar[acc], acc_phase, abort_flag, p.status, 35)) { ok = false; *abort_flag = 1; break; }
+      if (!warp_wait_or_abort(&tfull_bar[acc], acc_phase, abort_flag, p.status, 35)) { ok = false; *abort_flag = 1; break; }
       tc_fence_after();
       const uint32_t taddr0 = tmem_base + ((uint32_t)row_in_tile << 16) + (uint32_t)(acc * BN);
 #pragma unroll 1

@@ -166,7 +166,7 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
       const int tile = item / p.splits;
       tile_coords(tile, p.tiles_m, p.tiles_n, mb, nb_);
       const float4 bias = load_bias<BN, (MODE == EPI_F32 || MODE == EPI_F32_ANY) ? 32 : epi_group<BN>()>(p, nb_ * BN, half, lane);
-      if (!wait_or_abort(&tfull_bar[acc], acc_phase, abort_flag, p.status, 4)) { ok = false; *abort_flag = 1; break; }
+      if (!warp_wait_or_abort(&tfull_bar[acc], acc_phase, abort_flag, p.status, 4)) { ok = false; *abort_flag = 1; break; }
       tc_fence_after();
       const int row_in_tile = quarter * 32;
       const uint32_t taddr0 = tmem_base + ((uint32_t)row_in_tile << 16) + (uint32_t)(acc * BN);
@@ -377,7 +377,7 @@ gemm2_bf16_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant
       int mb, nb_;
       tile_coords(item / p.splits, p.tiles_m, p.tiles_n, mb, nb_);
       const float4 bias = load_bias<BN2, (MODE == EPI_F32 || MODE == EPI_F32_ANY) ? 32 : epi_group<BN2>()>(p, nb_ * BN2, half, lane);
-      if (!wait_or_abort(&tfull_bar[acc], acc_phase, abort_flag, p.status, 24)) { ok = false; *abort_flag = 1; break; }
+      if (!warp_wait_or_abort(&tfull_bar[acc], acc_phase, abort_flag, p.status, 24)) { ok = false; *abort_flag = 1; break; }
       tc_fence_after();
       const int row0 = mb * (2 * BM) + (int)rank * BM + quarter * 32;
       const uint32_t taddr0 = tmem_base + ((uint32_t)(quarter * 32) << 16) + (uint32_t)(acc * BN2);

@@ -401,6 +401,12 @@ __device__ __forceinline__ bool wait_or_abort(uint64_t* bar, uint32_t parity, vo
   report(status, NB_ST_MBAR_TIMEOUT, where, parity);
   return false;
 }
+// The same for a whole warp, whose lanes then exchange values (bias shuffles, staged rows): they go on or give up together.  A
+// lane that gave up alone, because the abort flag was set between two lanes' looks at it, would leave the others waiting.
+__device__ __forceinline__ bool warp_wait_or_abort(uint64_t* bar, uint32_t parity, volatile uint32_t* abort_flag, unsigned int* status,
+                                                   unsigned int where) {
+  return __all_sync(0xffffffffu, wait_or_abort(bar, parity, abort_flag, status, where));
+}
 
 // The four instructions of one k-block.  `ad` / `bd` are complete descriptors of the stage's operands, `astep` / `bstep` the
 // advance per instruction in descriptor units (16 bytes).  Nothing but additions stands between two instructions: with the

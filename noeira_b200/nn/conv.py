@@ -232,12 +232,13 @@ class BatchNorm2D(Module):
         self._stat = torch.empty(2 * self.c, dtype=torch.float32, device=x.device)
         mean = self._stat.data_ptr()
         lib = cuda_lib()
-        split = lib.nb_bn_split(ctypes.c_longlong(M))
+        # partial sums of the statistics: training only
+        part = _scratch(x.device, 2 * lib.nb_bn_split(ctypes.c_longlong(M)) * self.c).data_ptr() if self.training else None
         rc = residual.contiguous() if residual is not None else None
         check(lib.nb_bn_fwd(xc.data_ptr(), self.gamma.storage.data_ptr(), self.beta.storage.data_ptr(), None if rc is None else rc.data_ptr(),
                             y.data_ptr(), mean, mean + 4 * self.c,
                             self.running_mean.data.data_ptr(), self.running_var.data.data_ptr(),
-                            _scratch(x.device, 2 * split * self.c).data_ptr(), M, self.c, self.eps, self.momentum, int(self.relu),
+                            part, M, self.c, self.eps, self.momentum, int(self.relu),
                             int(self.training), raw_stream()), "bn_fwd")
         self._y = y
         return y
